@@ -35,9 +35,8 @@ std::vector<DeviceWords> g_words;
 // fastest on GB300: the mirror-quad gridder with 64 threads x 4 quads (shape
 // 22; 24 with 512-visibility tiles for S = 32) where 64 threads cover whole
 // quad columns (S/2 divides 64), else the Gauss pixel-pair shapes that make
-// whole passes for S = 24 (11) and 48 (12); the mirror-quad degridder with
-// kappa from shared memory, in column form (shape 32; 34 with its runs of
-// four quads for S = 32) or row by row (shape 31).
+// whole passes for S = 24 (11) and 48 (12); the tensor-core degridder (the last
+// shape, from S = 8 on).
 std::mutex g_shape_mutex;
 std::map<std::pair<int, int>, std::pair<int, int>> g_shapes;
 
@@ -51,8 +50,8 @@ int current_device() {
 // for at least four steps (S a multiple of 8, S >= 32), else the row form (31).
 std::pair<int, int> default_shapes(int S) {
     const int g = S == 32 ? 24 : (S >= 2 && 64 % (S / 2) == 0) ? 22 : S == 24 ? 11 : S == 48 ? 12 : 13;
-    const int d = S == 32 ? 34 : (S >= 32 && S % 8 == 0) ? 32 : 31;
-    return {g < gridder_fast_shapes() ? g : 0, d < degridder_fast_shapes() ? d : 0};
+    const int d = S >= 8 ? degridder_fast_shapes() - 1 : general_degridder_shape(S);
+    return {g, d};
 }
 
 std::pair<int, int> &shapes_of(int S) {
@@ -61,6 +60,11 @@ std::pair<int, int> &shapes_of(int S) {
     return it->second;
 }
 } // namespace
+
+// Degridder: the column form (32; 34 with its runs of four quads for S = 32)
+// where each lane's quads run down a column for at least four steps (S a
+// multiple of 8, S >= 32), else the row form (31).
+int general_degridder_shape(int S) { return S == 32 ? 34 : (S >= 32 && S % 8 == 0) ? 32 : 31; }
 
 int batched_gridder_shape(int S) {
     std::lock_guard<std::mutex> lock(g_shape_mutex);
@@ -178,8 +182,9 @@ int run_kernel(bool gridding, const idg_params *params, int variant, int64_t nr_
     if (int rc = device_words(&w)) return rc;
     a.status = w.status;
     if (variant == IDG_VARIANT_BATCHED) {
-        IDG_CUDA(cudaMemsetAsync(w.counter, 0, sizeof(int), st));
+        IDG_CUDA(cudaMemsetAsync(w.counter, 0, 3 * sizeof(int), st));
         a.work_counter = w.counter;
+        a.fallback = w.counter + 1;
     }
     cudaError_t e = gridding ? launch_gridder(a, variant, params->nr_channels, st)
                              : launch_degridder(a, variant, params->nr_channels, st);

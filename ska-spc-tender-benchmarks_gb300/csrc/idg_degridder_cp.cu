@@ -23,7 +23,7 @@
 // pixels: its MACs share each quad's phase factors (see its section).
 #include "idg_device.cuh"
 #include "idg_internal.h"
-#include "idg_ptx.cuh"
+#include "idg_tc.cuh"
 
 namespace idg {
 
@@ -634,8 +634,11 @@ __device__ __forceinline__ void column_loop_runs(f2 (&acc)[NPAIR][4][2], const K
 // COL: the column form (column_loop); otherwise quads row by row.
 // RUN > 0: the column form's runs of RUN quads as straight-line blocks, where
 // the batch's columns hold exactly kLanes * RUN quads.  PF: phasors first.
-template <int NT, int QB, int CB, int UNR, bool KSM, bool COL, int RUN, bool PF>
+// UNFIT: only the subgrids that the tensor-core degridder left (tc_fits).
+template <int NT, int QB, int CB, int UNR, bool KSM, bool COL, int RUN, bool PF, bool UNFIT>
 __device__ __forceinline__ void degridder_quad_body(const KernelArgs &a) {
+    __shared__ unsigned scratch[UNFIT ? 5 : 1];
+    if (UNFIT && a.fallback[0] == 0) return;
     constexpr int kT = NT, kCB = CB, kNP = CB / 2;
     static_assert(CB == 4 || CB == 8, "channel groups of 4 or 8");
     extern __shared__ __align__(16) unsigned char smem[];
@@ -670,6 +673,10 @@ __device__ __forceinline__ void degridder_quad_body(const KernelArgs &a) {
         if (!si.ok) {
             if (tid == 0) flag_status(a.status, kStatusBadPlan);
             continue;
+        }
+        if constexpr (UNFIT) {
+            TcSubgrid sg;
+            if (tc_fits<NT>(a, si, scratch, &sg, [] { __syncthreads(); })) continue;
         }
         const int nc = si.c1 - si.c0;
         const int ncb = (nc + kCB - 1) / kCB;
@@ -775,13 +782,13 @@ __device__ __forceinline__ void degridder_quad_body(const KernelArgs &a) {
 // The kernel: register budget from the CTAs per SM (MINB), or, with MAXR > 0,
 // a fixed cap of MAXR registers per thread (for CTA sizes whose budget the
 // compiler rounds down: 96-thread CTAs x 3 per SM may use 224 registers).
-template <int NT, int QB, int MINB, int CB, int UNR, bool KSM, bool COL, int RUN, bool PF>
+template <int NT, int QB, int MINB, int CB, int UNR, bool KSM, bool COL, int RUN, bool PF, bool UNFIT>
 __global__ void __launch_bounds__(NT, MINB) degridder_quad_kernel(KernelArgs a) {
-    degridder_quad_body<NT, QB, CB, UNR, KSM, COL, RUN, PF>(a);
+    degridder_quad_body<NT, QB, CB, UNR, KSM, COL, RUN, PF, UNFIT>(a);
 }
 template <int MAXR, int NT, int QB, int CB, int UNR, bool KSM, bool COL, int RUN, bool PF>
 __global__ void __maxnreg__(MAXR) degridder_quad_kernel_r(KernelArgs a) {
-    degridder_quad_body<NT, QB, CB, UNR, KSM, COL, RUN, PF>(a);
+    degridder_quad_body<NT, QB, CB, UNR, KSM, COL, RUN, PF, false>(a);
 }
 
 // ---------------------------------------------------------------------------
@@ -1070,14 +1077,14 @@ cudaError_t launch_oct(const KernelArgs &a, cudaStream_t stream) {
 }
 
 template <int NT, int QB, int MINB, int CB, int UNR, bool KSM = false, bool COL = false, int RUN = 0, bool PF = false,
-          int MAXR = 0>
+          int MAXR = 0, bool UNFIT = false>
 cudaError_t launch_quad(const KernelArgs &a, cudaStream_t stream) {
     if (a.S % 2 != 0) return cudaErrorInvalidValue;
     void (*kern)(KernelArgs);
     if constexpr (MAXR > 0)
         kern = degridder_quad_kernel_r<MAXR, NT, QB, CB, UNR, KSM, COL, RUN, PF>;
     else
-        kern = degridder_quad_kernel<NT, QB, MINB, CB, UNR, KSM, COL, RUN, PF>;
+        kern = degridder_quad_kernel<NT, QB, MINB, CB, UNR, KSM, COL, RUN, PF, UNFIT>;
     const size_t smem = quad_layout(a.S, a.C, QB).total;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
@@ -1153,6 +1160,17 @@ cudaError_t launch_degridder_cp(const KernelArgs &a, cudaStream_t stream, int sh
     case 12: return launch_cp<128, 512, 2, 8, kGaussCp, 8>(a, stream);
     default: return launch_cp<128, 256, 4, 8, 0, 1>(a, stream);
     }
+}
+
+// The subgrids that the tensor-core degridder left, in the form that is
+// fastest for the size without it (the plan entries that it flagged are skipped
+// again; with nothing left every CTA returns at once).
+cudaError_t launch_degridder_unfit(const KernelArgs &args, cudaStream_t stream) {
+    KernelArgs a = args;
+    a.work_counter = a.fallback + 1;
+    if (a.S == 32) return launch_quad<128, 256, 2, 8, 1, true, true, 4, false, 0, true>(a, stream);
+    if (a.S > 32 && a.S % 8 == 0) return launch_quad<128, 256, 2, 8, 1, true, true, 0, false, 0, true>(a, stream);
+    return launch_quad<128, 256, 3, 8, 1, true, false, 0, false, 0, true>(a, stream);
 }
 
 } // namespace idg

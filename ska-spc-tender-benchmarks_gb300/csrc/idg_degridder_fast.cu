@@ -386,9 +386,14 @@ cudaError_t launch_shape(const KernelArgs &a, cudaStream_t stream) {
 
 // Launch shapes of the batched degridder (index = shape id).
 // Shapes 0-14 are the pixel-pair kernel above; 15 and up the channel-pair kernel.
-int degridder_fast_shapes() { return 15 + degridder_cp_shapes(); }
+// The last one is the tensor-core kernel (idg_degridder_tc.cu) where it applies.
+int degridder_fast_shapes() { return 16 + degridder_cp_shapes(); }
 
 cudaError_t launch_degridder_fast(const KernelArgs &a, cudaStream_t stream, int shape) {
+    if (shape == 15 + degridder_cp_shapes()) {
+        if (a.fallback && degridder_tc_supported(a.S, a.image_size)) return launch_degridder_tc(a, stream);
+        shape = general_degridder_shape(a.S);
+    }
     if (shape >= 15) return launch_degridder_cp(a, stream, shape - 15);
     switch (shape) {
     case 1: return launch_shape<128, 512, 4>(a, stream); // 16 warps/SM, register cap 128

@@ -101,6 +101,15 @@ __device__ __forceinline__ void load_jones(const float4 *base, cf *j) {
     j[3] = {b.z, b.w};
 }
 
+// Constants of a tensor-core launch (idg_tc.cuh), from the host.
+struct TcConst {
+    float f_max, eps_per_g;  // f at the edge pixel; radians of d c at the corner pixel per turn of d
+    float turns_per_step;    // turns per pixel, metre and unit wavenumber
+    float s2h, s2l;          // a quarter of the squared pixel size, hi + lo
+    float d2h, d2l, i2h, i2l; // metres to turns per pixel step; 1 / 2 pi; hi + lo
+    float f[32], cx[32];     // f and cx of the pixels outward from the centre
+};
+
 // Everything a kernel needs about one call, by value in the launch.
 struct KernelArgs {
     int G, S, C, nr_stations, nr_aterms, nr_w_planes;
@@ -120,6 +129,8 @@ struct KernelArgs {
     unsigned *status;     // device check word (may be NULL)
     int max_ctas;         // persistent kernels: at most this many CTAs (0 = fill the GPU)
     int share_den;        // persistent kernels: 1/share_den of the CTAs that fill the GPU (0, 1 = all)
+    int *fallback;        // tensor-core kernels: [0] subgrids left to the general kernel, [1] its work counter
+    TcConst tc;           // tensor-core kernels: constants of the launch
 };
 
 // Plan entry after validation.

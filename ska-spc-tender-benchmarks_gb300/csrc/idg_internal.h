@@ -26,6 +26,13 @@ int degridder_fast_shapes();
 // Channel-pair-packed batched degridder (idg_degridder_cp.cu), shapes 0..degridder_cp_shapes()-1.
 cudaError_t launch_degridder_cp(const KernelArgs &a, cudaStream_t stream, int shape);
 int degridder_cp_shapes();
+// Tensor-core degridder (idg_degridder_tc.cu; needs a.fallback): the subgrids its
+// expansion does not hold for go to the general kernel behind it.
+bool degridder_tc_supported(int S, double image_size);
+cudaError_t launch_degridder_tc(const KernelArgs &a, cudaStream_t stream);
+cudaError_t launch_degridder_unfit(const KernelArgs &a, cudaStream_t stream);
+// The shape for subgrid size S among the kernels that take any geometry.
+int general_degridder_shape(int S);
 int batched_degridder_shape(int S);
 void set_batched_degridder_shape(int S, int shape);
 

@@ -29,7 +29,8 @@ struct idg_plan {
     idg_metadata *d_md = nullptr;
     idg_subgrid_ext *d_ext = nullptr;
     int *d_work = nullptr;
-    unsigned *d_words = nullptr; // [0] gridder counter, [1] degridder counter, [2] check word
+    // [2] check word; [16..18] gridder counter, subgrids left to the general kernel, its counter; [32..34] degridder's
+    unsigned *d_words = nullptr;
     void *d_subgrids = nullptr;
     void *bins_mem = nullptr; // the adder's tile bins (and their own metadata copy)
     idg::TileBinsDev bins;
@@ -80,7 +81,8 @@ KernelArgs plan_args(const idg_plan *p, const float *uvw, const float *k, const 
     a.vis = reinterpret_cast<float4 *>(vis);
     a.subgrids = reinterpret_cast<float2 *>(subgrids);
     a.work_list = p->d_work;
-    a.work_counter = reinterpret_cast<int *>(p->d_words) + (degrid ? 1 : 0);
+    a.work_counter = reinterpret_cast<int *>(p->d_words) + (degrid ? 32 : 16);
+    a.fallback = a.work_counter + 1;
     a.status = p->d_words + 2;
     a.max_ctas = p->max_ctas;
     return a;
@@ -103,7 +105,7 @@ int check_data(const idg_plan *p, const float *uvw, const float *k, const void *
 int grid_step(idg_plan *p, const float *uvw, const float *k, const void *vis, const float *taper, const void *aterms,
               void *grid, cudaStream_t st) {
     const idg_params &q = p->params;
-    if (p->variant == IDG_VARIANT_BATCHED) IDG_CUDA(cudaMemsetAsync(p->d_words, 0, sizeof(int), st));
+    if (p->variant == IDG_VARIANT_BATCHED) IDG_CUDA(cudaMemsetAsync(p->d_words + 16, 0, 3 * sizeof(int), st));
     KernelArgs a = plan_args(p, uvw, k, taper, aterms, const_cast<void *>(vis), p->d_subgrids, false);
     cudaError_t e = launch_gridder(a, p->variant, q.nr_channels, st);
     if (e != cudaSuccess) return cuda_fail(e, "plan gridder");
@@ -124,7 +126,7 @@ int degrid_step(idg_plan *p, const float *uvw, const float *k, void *vis_out, co
                                      reinterpret_cast<float2 *>(p->d_subgrids), taper, st);
     if (e != cudaSuccess) return cuda_fail(e, "plan split + subgrid fft");
     if (p->variant == IDG_VARIANT_BATCHED)
-        IDG_CUDA(cudaMemsetAsync(reinterpret_cast<int *>(p->d_words) + 1, 0, sizeof(int), st));
+        IDG_CUDA(cudaMemsetAsync(p->d_words + 32, 0, 3 * sizeof(int), st));
     KernelArgs a = plan_args(p, uvw, k, taper, aterms, vis_out, p->d_subgrids, true);
     e = launch_degridder(a, p->variant, q.nr_channels, st);
     if (e != cudaSuccess) return cuda_fail(e, "plan degridder");

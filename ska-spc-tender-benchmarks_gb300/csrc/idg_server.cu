@@ -239,6 +239,7 @@ void idg_server::launch(Job &j) {
     a.work_list = static_cast<const int *>(dp(L.work));
     a.work_counter = static_cast<int *>(dp(L.words));
     a.status = static_cast<unsigned *>(dp(L.words)) + 2;
+    a.fallback = static_cast<int *>(dp(L.words)) + 4;
     // Running jobs share the SMs: a persistent kernel takes 1/share of the
     // CTAs that would fill the GPU with its own launch shape, and keeps them
     // to its end.  Peers estimated to finish within a quarter of this job's
