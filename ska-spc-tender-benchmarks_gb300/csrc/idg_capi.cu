@@ -31,12 +31,8 @@ std::mutex g_words_mutex;
 std::vector<DeviceWords> g_words;
 
 // Launch shapes of the batched kernels per (device, subgrid size), set by the
-// autotuner or by idg_set_batched_shapes().  Until then, the shapes measured
-// fastest on GB300: the mirror-quad gridder with 64 threads x 4 quads (shape
-// 22; 24 with 512-visibility tiles for S = 32) where 64 threads cover whole
-// quad columns (S/2 divides 64), else the Gauss pixel-pair shapes that make
-// whole passes for S = 24 (11) and 48 (12); the tensor-core degridder (the last
-// shape, from S = 8 on).
+// autotuner or by idg_set_batched_shapes().  Until then the tensor-core kernels
+// (the last shape of each) from S = 8 on.
 std::mutex g_shape_mutex;
 std::map<std::pair<int, int>, std::pair<int, int>> g_shapes;
 
@@ -49,7 +45,7 @@ int current_device() {
 // Degridder: the column form (32) where each lane's quads run down a column
 // for at least four steps (S a multiple of 8, S >= 32), else the row form (31).
 std::pair<int, int> default_shapes(int S) {
-    const int g = S == 32 ? 24 : (S >= 2 && 64 % (S / 2) == 0) ? 22 : S == 24 ? 11 : S == 48 ? 12 : 13;
+    const int g = S >= 8 ? gridder_fast_shapes() - 1 : general_gridder_shape(S);
     const int d = S >= 8 ? degridder_fast_shapes() - 1 : general_degridder_shape(S);
     return {g, d};
 }
@@ -61,6 +57,13 @@ std::pair<int, int> &shapes_of(int S) {
 }
 } // namespace
 
+// Without the tensor cores: the mirror-quad gridder with 64 threads x 4 quads
+// (22; 24 with 512-visibility tiles for S = 32) where 64 threads cover whole
+// quad columns (S/2 divides 64), else the Gauss pixel-pair shapes that make
+// whole passes for S = 24 (11) and 48 (12).
+int general_gridder_shape(int S) {
+    return S == 32 ? 24 : (S >= 2 && 64 % (S / 2) == 0) ? 22 : S == 24 ? 11 : S == 48 ? 12 : 13;
+}
 // Degridder: the column form (32; 34 with its runs of four quads for S = 32)
 // where each lane's quads run down a column for at least four steps (S a
 // multiple of 8, S >= 32), else the row form (31).

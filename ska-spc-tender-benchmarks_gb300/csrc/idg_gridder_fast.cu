@@ -24,7 +24,7 @@
 //    when they are faster on the data at hand.
 #include "idg_device.cuh"
 #include "idg_internal.h"
-#include "idg_ptx.cuh"
+#include "idg_tc.cuh"
 
 namespace idg {
 
@@ -402,8 +402,11 @@ __device__ __forceinline__ bool stage_tile(const KernelArgs &a, const SubgridInf
 
 // Kernel shape: NT threads per CTA, PAIRS pixel pairs per thread per pass,
 // TV visibilities per staged tile, at least MINB CTAs per SM (register cap).
-template <int NT, int PAIRS, int TV, int MINB, int PIPE>
+// UNFIT: only the subgrids that the tensor-core gridder left (tc_fits).
+template <int NT, int PAIRS, int TV, int MINB, int PIPE, bool UNFIT>
 __global__ void __launch_bounds__(NT, MINB) gridder_fast_kernel(KernelArgs a) {
+    __shared__ unsigned scratch[UNFIT ? 5 : 1];
+    if (UNFIT && a.fallback[0] == 0) return;
     constexpr int kT = NT, kPairs = PAIRS, kPassPairs = NT * PAIRS, kTileVis = TV, kMaxChunk = TV;
     constexpr bool kG = (PIPE & kGauss) != 0;
     constexpr int kAcc = kG ? 12 : 8, kUnr = (PIPE & kUnroll4) ? 4 : (PIPE & kUnroll2) ? 2 : 1;
@@ -454,6 +457,10 @@ __global__ void __launch_bounds__(NT, MINB) gridder_fast_kernel(KernelArgs a) {
             if (tid == 0) flag_status(a.status, kStatusBadPlan);
             for (int i = tid; i < 4 * S2; i += kT) a.subgrids[(size_t)s * 4 * S2 + i] = make_float2(0.f, 0.f);
             continue;
+        }
+        if constexpr (UNFIT) {
+            TcSubgrid sg;
+            if (tc_fits<NT>(a, si, scratch, &sg, [] { __syncthreads(); })) continue;
         }
         // channel offsets relative to the middle channel; max |kappa|
         const int cref = si.c0 + (nc > 0 ? (nc - 1) / 2 : 0);
@@ -702,8 +709,10 @@ __device__ __forceinline__ void quad_tile(f2 (&acc)[GP][4][8], const f2 *qg, con
 // Kernel of the mirror-quad form: NT threads, GP quad pairs per thread per
 // pass, TV visibilities per staged tile, at least MINB CTAs per SM.  Staging,
 // coefficients, work distribution and failure handling as gridder_fast_kernel.
-template <int NT, int GP, int TV, int MINB, int UNR>
+template <int NT, int GP, int TV, int MINB, int UNR, bool UNFIT>
 __global__ void __launch_bounds__(NT, MINB) gridder_quad_kernel(KernelArgs a) {
+    __shared__ unsigned scratch[UNFIT ? 5 : 1];
+    if (UNFIT && a.fallback[0] == 0) return;
     constexpr int kT = NT, kPassQuads = NT * GP * 2, kTileVis = TV, kMaxChunk = TV;
     extern __shared__ __align__(16) unsigned char smem[];
     const int S = a.S, S2 = S * S, Sh = S / 2, nquads = Sh * Sh;
@@ -744,6 +753,10 @@ __global__ void __launch_bounds__(NT, MINB) gridder_quad_kernel(KernelArgs a) {
             if (tid == 0) flag_status(a.status, kStatusBadPlan);
             for (int i = tid; i < 4 * S2; i += kT) a.subgrids[(size_t)s * 4 * S2 + i] = make_float2(0.f, 0.f);
             continue;
+        }
+        if constexpr (UNFIT) {
+            TcSubgrid sg;
+            if (tc_fits<NT>(a, si, scratch, &sg, [] { __syncthreads(); })) continue;
         }
         const int cref = si.c0 + (nc > 0 ? (nc - 1) / 2 : 0);
         const double kref = nc > 0 ? (double)a.wavenumbers[cref] : 0.0;
@@ -908,12 +921,13 @@ __global__ void __launch_bounds__(NT, MINB) gridder_quad_kernel(KernelArgs a) {
 //  22: shape 20 with the channel loop unrolled by four
 //  23: shape 22 with 384-visibility tiles (fewer stages per subgrid)
 //  24: shape 22 with 512-visibility tiles
+//  25: the tensor-core kernel (idg_gridder_tc.cu) where it applies, else general_gridder_shape()
 // load_only: only make sure the kernel is loaded into the current context
 // (under lazy module loading a kernel is otherwise loaded, which takes device
 // memory, at its first launch).
-template <int NT, int PAIRS, int TV, int MINB, int PIPE>
+template <int NT, int PAIRS, int TV, int MINB, int PIPE, bool UNFIT = false>
 cudaError_t launch_shape(const KernelArgs &a, cudaStream_t stream, bool load_only) {
-    auto kern = gridder_fast_kernel<NT, PAIRS, TV, MINB, PIPE>;
+    auto kern = gridder_fast_kernel<NT, PAIRS, TV, MINB, PIPE, UNFIT>;
     if (load_only) {
         cudaFuncAttributes fa;
         return cudaFuncGetAttributes(&fa, kern);
@@ -935,9 +949,9 @@ cudaError_t launch_shape(const KernelArgs &a, cudaStream_t stream, bool load_onl
     return cudaGetLastError();
 }
 
-template <int NT, int GP, int TV, int MINB, int UNR>
+template <int NT, int GP, int TV, int MINB, int UNR, bool UNFIT = false>
 cudaError_t launch_quad(const KernelArgs &a, cudaStream_t stream, bool load_only) {
-    auto kern = gridder_quad_kernel<NT, GP, TV, MINB, UNR>;
+    auto kern = gridder_quad_kernel<NT, GP, TV, MINB, UNR, UNFIT>;
     if (load_only) {
         cudaFuncAttributes fa;
         return cudaFuncGetAttributes(&fa, kern);
@@ -962,10 +976,17 @@ cudaError_t launch_quad(const KernelArgs &a, cudaStream_t stream, bool load_only
 
 } // namespace
 
-int gridder_fast_shapes() { return 25; }
+int gridder_fast_shapes() { return 26; }
 
 namespace {
 cudaError_t dispatch_gridder_fast(const KernelArgs &a, cudaStream_t stream, int shape, bool load_only) {
+    if (shape == 25) {
+        if (load_only) return load_gridder_tc();
+        // the test of a lost copy needs a kernel that stages by bulk copies
+        if (a.fallback && gridder_tc_supported(a.S, a.image_size) && !(a.flags & IDG_FLAG_TEST_LOST_COPY))
+            return launch_gridder_tc(a, stream);
+        shape = general_gridder_shape(a.S);
+    }
     switch (shape) {
     case 1: return launch_shape<128, 4, 256, 2, 1>(a, stream, load_only);
     case 2: return launch_shape<128, 2, 128, 4, 1>(a, stream, load_only);
@@ -998,6 +1019,27 @@ cudaError_t dispatch_gridder_fast(const KernelArgs &a, cudaStream_t stream, int 
 
 cudaError_t launch_gridder_fast(const KernelArgs &a, cudaStream_t stream, int shape) {
     return dispatch_gridder_fast(a, stream, shape, false);
+}
+
+// The subgrids that the tensor-core gridder left, in the form that is fastest
+// for the size without it (with nothing left every CTA returns at once).
+cudaError_t launch_gridder_unfit(const KernelArgs &args, cudaStream_t stream, bool load_only) {
+    KernelArgs a = args;
+    if (load_only) {
+        if (cudaError_t e = launch_quad<64, 2, 512, 4, 4, true>(a, stream, true)) return e;
+        if (cudaError_t e = launch_quad<64, 2, 256, 4, 4, true>(a, stream, true)) return e;
+        if (cudaError_t e = launch_shape<96, 3, 256, 3, kGauss | kPipe | kUnroll2, true>(a, stream, true)) return e;
+        if (cudaError_t e = launch_shape<128, 3, 256, 2, kGauss | kPipe | kUnroll2, true>(a, stream, true)) return e;
+        return launch_shape<128, 4, 256, 2, kGauss | kPipe | kUnroll4, true>(a, stream, true);
+    }
+    a.work_counter = a.fallback + 1;
+    switch (general_gridder_shape(a.S)) {
+    case 24: return launch_quad<64, 2, 512, 4, 4, true>(a, stream, false);
+    case 22: return launch_quad<64, 2, 256, 4, 4, true>(a, stream, false);
+    case 11: return launch_shape<96, 3, 256, 3, kGauss | kPipe | kUnroll2, true>(a, stream, false);
+    case 12: return launch_shape<128, 3, 256, 2, kGauss | kPipe | kUnroll2, true>(a, stream, false);
+    default: return launch_shape<128, 4, 256, 2, kGauss | kPipe | kUnroll4, true>(a, stream, false);
+    }
 }
 
 cudaError_t load_gridder_fast() {

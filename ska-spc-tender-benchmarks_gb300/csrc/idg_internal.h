@@ -15,6 +15,14 @@ cudaError_t launch_degridder(const KernelArgs &a, int variant, int max_nc, cudaS
 // shape: index into the batched gridder's launch shapes (see gridder_fast_shapes()).
 cudaError_t launch_gridder_fast(const KernelArgs &a, cudaStream_t stream, int shape);
 int gridder_fast_shapes();
+// Tensor-core gridder (idg_gridder_tc.cu; needs a.fallback): the subgrids its
+// expansion does not hold for go to the general kernel behind it.
+bool gridder_tc_supported(int S, double image_size);
+cudaError_t launch_gridder_tc(const KernelArgs &a, cudaStream_t stream);
+cudaError_t load_gridder_tc();
+cudaError_t launch_gridder_unfit(const KernelArgs &a, cudaStream_t stream, bool load_only);
+// The shape for subgrid size S among the kernels that take any geometry.
+int general_gridder_shape(int S);
 // Loads the kernels of every batched gridder shape into the current device's
 // context without launching them.
 cudaError_t load_gridder_fast();

@@ -1,10 +1,11 @@
 // idg_noalloc.cu -- the batched gridder for callers that may not allocate
 // device memory.
 //
-// The batched gridder needs two words of device scratch: the work counter its
-// persistent CTAs pull subgrids from, and the check word it flags bad plan
-// entries in.  idg_gridder() keeps those words in memory the library obtains
-// with cudaMalloc on first use.  Some callers cannot allow that: a host
+// The batched gridder needs four words of device scratch: the work counter its
+// persistent CTAs pull subgrids from, the check word it flags bad plan entries
+// in, and the two words by which its tensor-core and general kernels hand over.
+// idg_gridder() keeps those words in memory the library obtains with cudaMalloc
+// on first use.  Some callers cannot allow that: a host
 // application that has reserved all device memory through its own pool, a
 // framework that forbids allocations outside its allocator, or a real-time
 // loop that must not allocate once it is running.  idg_gridder_noalloc() runs
@@ -13,9 +14,9 @@
 //
 // The array is g_noalloc_scratch: 256 bytes, loaded with the library on every
 // device that uses it and kept until the process exits.  Word 0 is the work
-// counter, word 1 the check word.  Each call clears both on the caller's
-// stream before the launch.  All calls on a device share the array, so calls
-// whose kernels overlap on the GPU (other streams, no ordering between them)
+// counter, word 1 the check word, words 2 and 3 the hand-over.  Each call clears
+// them on the caller's stream before the launch.  All calls on a device share
+// the array, so calls whose kernels overlap on the GPU (other streams, no ordering between them)
 // race on the work counter and must be serialised by the caller.  A plan
 // entry the kernel rejects yields an all-zero subgrid and sets bit 0 of the
 // check word, which idg_noalloc_status() reads (idg_device_status() reports
@@ -96,7 +97,7 @@ extern "C" IDG_API int idg_gridder_noalloc(const idg_params *params, int64_t nr_
         return fail(IDG_ERR_INVALID_ARGUMENT, "visibilities, aterms and subgrids must be 16-byte aligned");
 
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    IDG_CUDA(cudaMemsetAsync(scratch, 0, 2 * sizeof(unsigned int), st));
+    IDG_CUDA(cudaMemsetAsync(scratch, 0, 4 * sizeof(unsigned int), st));
 
     KernelArgs a{};
     a.G = params->grid_size;
@@ -120,6 +121,7 @@ extern "C" IDG_API int idg_gridder_noalloc(const idg_params *params, int64_t nr_
     a.subgrids = reinterpret_cast<float2 *>(subgrids);
     a.work_counter = reinterpret_cast<int *>(scratch);
     a.status = reinterpret_cast<unsigned *>(scratch) + 1;
+    a.fallback = reinterpret_cast<int *>(scratch) + 2;
     cudaError_t e = launch_gridder_fast(a, st, batched_gridder_shape(a.S));
     if (e != cudaSuccess) return cuda_fail(e, "allocation-free gridder launch");
     return IDG_OK;

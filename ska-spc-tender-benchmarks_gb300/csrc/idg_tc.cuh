@@ -262,6 +262,8 @@ __device__ __forceinline__ float tc_scale(unsigned max_bits, float &inv) {
 // by 1.6e-7 to 2.1e-7 (measured against 64 bits, whatever the lengths); this
 // factor puts the mean of it back.
 constexpr float kTcTruncation = 1.f + 2.384185791015625e-7f; // 1 + 2^-22
+// The gridder's accumulators take four full-size products per stage.
+constexpr float kTcTruncationPerStage = 1.0e-7f;
 
 // Bounded wait; on expiry raises the CTA's abort flag and the status bit, after
 // which every wait returns at once: the roles run to their next common check

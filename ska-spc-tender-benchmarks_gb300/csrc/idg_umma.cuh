@@ -60,6 +60,16 @@ __device__ __forceinline__ void umma_f16_ts(uint32_t d, uint32_t a, uint32_t b_l
         "r"(a), "r"(b_lo), "r"(lead), "n"(ACC ? 1 : 0), "r"(IDESC), "r"(DESC_HI)
         : "memory");
 }
+// The same with the choice at run time.
+template <uint32_t IDESC, uint32_t DESC_HI>
+__device__ __forceinline__ void umma_f16_ts_if(uint32_t d, uint32_t a, uint32_t b_lo, uint32_t acc, uint32_t lead) {
+    asm volatile(
+        "{\n .reg .pred p, q;\n .reg .b64 b;\n setp.ne.u32 q, %3, 0;\n setp.ne.u32 p, %4, 0;\n"
+        " mov.b64 b, {%2, %6};\n"
+        " @q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %5, p;\n}\n" ::"r"(d),
+        "r"(a), "r"(b_lo), "r"(lead), "r"(acc), "r"(IDESC), "r"(DESC_HI)
+        : "memory");
+}
 // The mbarrier completes a phase when every MMA issued so far by this thread has finished.
 __device__ __forceinline__ void umma_commit(uint64_t *bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_addr(bar))
@@ -74,6 +84,19 @@ __device__ __forceinline__ void umma_commit(uint64_t *bar) {
 __device__ __forceinline__ void tmem_st4(uint32_t addr, const uint32_t (&r)[4]) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(r[0]), "r"(r[1]),
                  "r"(r[2]), "r"(r[3]));
+}
+// 16 columns, arrived when this returns.
+__device__ __forceinline__ void tmem_ld16(uint32_t addr, f2 (&v)[8]) {
+    uint32_t r[16];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
+        "%15}, [%16];\n"
+        "tcgen05.wait::ld.sync.aligned;"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(addr));
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = (f2)r[2 * i] | ((f2)r[2 * i + 1] << 32);
 }
 // Two runs of 16 columns, arrived when this returns (the wait is part of the
 // statement, so nothing that uses the registers can move before it).

@@ -58,6 +58,15 @@ def _degrid(c, oracle_mod, name, tol, scale=1.0):
     check_rel(f"degridder {name}", got.astype(np.complex128) / np.float64(np.float32(scale)), want, tol)
 
 
+def _grid(c, oracle_mod, name, tol, scale=1.0):
+    sp = spec_for(c["G"], c["S"], c["C"], c["ns"], 1, c["img"])
+    prm = oracle_mod.params(c["G"], c["S"], c["C"], c["ns"], len(c["md"]), c["img"])
+    got = grid_gpu(sp, c["md"], c["uvw"], c["k"], c["vis"] * np.float32(scale), c["taper"], c["at"],
+                   L.VARIANT_BATCHED)
+    want = oracle_mod.gridder(prm, c["uvw"], c["k"], c["vis"], c["taper"], c["at"], c["md"])
+    check_rel(f"gridder {name}", got.astype(np.complex128) / np.float64(np.float32(scale)), want, tol)
+
+
 # lengths x channels: one visibility, and one below, at and above 16, 32, 128 and 256
 EDGES = [([1, 2, 5], 3), ([16, 17, 31, 32, 33], 1), ([127, 128, 129], 1), ([8, 15, 17], 16), ([3], 100)]
 
@@ -138,3 +147,58 @@ def test_degridder_equals_the_general_kernel(idg, S):
     args = (sp, c["md"], c["uvw"], c["k"], c["sub"], c["taper"], c["at"], c["uvw"].shape[0], L.VARIANT_BATCHED)
     here, general = _both(S, args, degrid_gpu, 31, False)
     check_rel(f"degridder S={S} against the general kernel", here, general, TOL + 1e-6)
+
+
+@pytest.mark.parametrize("S", [8, 10, 16, 18, 24, 30, 32, 34, 48, 50, 64])
+def test_gridder_block_and_chunk_edges(oracle_mod, idg, S):
+    for i, (lengths, C) in enumerate(EDGES):
+        _grid(_case(S, lengths, C, seed=200 * S + i), oracle_mod, f"S={S} {lengths}x{C}", TOL)
+
+
+@pytest.mark.parametrize("image_size", [0.05, 0.2])
+def test_gridder_wide_w(oracle_mod, idg, image_size):
+    _grid(_wide(image_size), oracle_mod, f"wide w, image {image_size}", TOL_GENERAL)
+
+
+def test_gridder_image_too_wide_is_the_general_kernel(idg):
+    c = _wide(0.5)
+    sp = spec_for(c["G"], 32, 8, c["ns"], 1, c["img"])
+    here, general = _both(32, (sp, c["md"], c["uvw"], c["k"], c["vis"], c["taper"], c["at"], L.VARIANT_BATCHED),
+                          grid_gpu, 24, True)
+    assert np.array_equal(here, general)
+
+
+@pytest.mark.parametrize("scale", [0.0, 1e-30, 1e-12, 1e12, 1e30])
+def test_gridder_magnitudes(oracle_mod, idg, scale):
+    c = _case(24, [20, 33], 7, seed=9)
+    if scale == 0.0:
+        sp = spec_for(c["G"], 24, 7, c["ns"], 1, c["img"])
+        assert not grid_gpu(sp, c["md"], c["uvw"], c["k"], 0 * c["vis"], c["taper"], c["at"], L.VARIANT_BATCHED).any()
+    else:
+        _grid(c, oracle_mod, f"scale {scale}", TOL, scale)
+
+
+def test_gridder_chunks_of_very_different_magnitude(oracle_mod, idg):
+    """Chunks of 128 visibilities carry scales of their own."""
+    c = _case(32, [256], 4, seed=12)
+    c["vis"] *= (10.0 ** np.linspace(-9, 9, 256)).astype(np.float32)[:, None, None]
+    _grid(c, oracle_mod, "mixed magnitudes", TOL)
+
+
+def test_gridder_values_that_are_not_finite(idg):
+    """A NaN or infinity in a visibility reaches its own subgrid and no others."""
+    c = _case(32, [20, 20, 20], 4, seed=4)
+    c["vis"][25, 2, 1] = np.nan
+    c["vis"][59, 0, 3] = np.inf
+    sp = spec_for(c["G"], 32, 4, c["ns"], 1, c["img"])
+    got = grid_gpu(sp, c["md"], c["uvw"], c["k"], c["vis"], c["taper"], c["at"], L.VARIANT_BATCHED)
+    assert np.isfinite(got[0]).all() and not np.isfinite(got[1]).all() and not np.isfinite(got[2]).all()
+
+
+@pytest.mark.parametrize("S", [16, 24, 32, 64])
+def test_gridder_equals_the_general_kernel(idg, S):
+    c = _case(S, [37, 64, 5], 9, seed=S)
+    sp = spec_for(c["G"], S, 9, c["ns"], 1, c["img"])
+    args = (sp, c["md"], c["uvw"], c["k"], c["vis"], c["taper"], c["at"], L.VARIANT_BATCHED)
+    here, general = _both(S, args, grid_gpu, 13, True)
+    check_rel(f"gridder S={S} against the general kernel", here, general, TOL + 1e-6)
