@@ -28,12 +28,15 @@
 //    one for the sums and the epilogue, two warps that bring in the chunks, one
 //    that issues the products, one that looks for the next subgrid.
 // One CTA of 20 warps per SM and all of its tensor memory.
-// Measured on GB300, 4,416 subgrids of 128 x 16 visibilities at S = 32: 1.49 ms
-// (46 SM cycles per visibility) against 5.02 ms for the mirror-quad kernel.  The
-// products take 16 of those cycles; shared memory bounds the rest (73 % of its
-// wavefronts: every factor warp reads every visibility, and with neighbouring
-// lanes on different visibilities a 16-byte read takes four).  28 subgrids of
-// 64 x 16 in one call: 41 us against 213 us.
+// Measured on GB300, 4,416 subgrids of 128 x 16 visibilities at S = 32: 1.38 ms
+// (43 SM cycles per visibility) against 5.02 ms for the mirror-quad kernel.  The
+// products take 16 of those cycles; shared memory (73 % of its wavefronts: every
+// factor warp reads every visibility, and with neighbouring lanes on different
+// visibilities a 16-byte read takes four) and the issue slots bound the rest.
+// The roles run five different loops on one SM, so these are kept small: with
+// the half stages unrolled and two stages of x-factors at a time, the same work
+// missed the instruction cache and took 1.47 ms.  28 subgrids of 64 x 16 in one
+// call: 42 us against 213 us.
 #include "idg_tc.cuh"
 #include "idg_internal.h"
 
@@ -197,34 +200,29 @@ __device__ __forceinline__ Raw load_raw(const KernelArgs &a, const float4 *chan,
     return r;
 }
 
-// x-factors of NS consecutive stages (two at a time keep more independent work
-// in flight): thread (x = lane, eight visibilities of warp w in each).
-template <int XR, int NS>
-__device__ __forceinline__ void make_b(unsigned char *b, uint32_t gs, const ChunkData &cd, int v0, f2 H, f2 F, f2 CX,
-                                       bool cross, int lane, int w) {
-    uint32_t ch[NS][4], cl[NS][4], sh[NS][4], sl[NS][4], c1[NS][4], s1[NS][4];
+// x-factors of one stage: thread (x = lane, eight visibilities of warp w).
+template <int XR>
+__device__ __forceinline__ void make_b(unsigned char *slot, const ChunkData &cd, int v0, f2 H, f2 F, f2 CX, bool cross,
+                                       int lane, int w) {
+    uint32_t ch[4], cl[4], sh[4], sl[4], c1[4], s1[4];
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
+        const float4 hi = *reinterpret_cast<const float4 *>(&cd.ah[v0 + 4 * q]);
+        const float4 lo = *reinterpret_cast<const float4 *>(&cd.al[v0 + 4 * q]);
+        const float4 d = *reinterpret_cast<const float4 *>(&cd.d[v0 + 4 * q]);
 #pragma unroll
-        for (int n = 0; n < NS; ++n) {
-            const int v = v0 + n * kStage + 4 * q;
-            const float4 hi = *reinterpret_cast<const float4 *>(&cd.ah[v]);
-            const float4 lo = *reinterpret_cast<const float4 *>(&cd.al[v]);
-            const float4 d = *reinterpret_cast<const float4 *>(&cd.d[v]);
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const int i = 2 * q + e;
-                const f2 D = e ? pack2(d.z, d.w) : pack2(d.x, d.y);
-                f2 c, s;
-                tc_sincos(e ? pack2(hi.z, hi.w) : pack2(hi.x, hi.y), e ? pack2(lo.z, lo.w) : pack2(lo.x, lo.y), D, H,
-                          F, c, s);
-                tc_split(c, ch[n][i], cl[n][i]);
-                tc_split(s, sh[n][i], sl[n][i]);
-                if (cross) {
-                    const f2 x = fmul2(D, CX);
-                    c1[n][i] = tc_half2(fmul2(c, x));
-                    s1[n][i] = tc_half2(fmul2(s, x));
-                }
+        for (int e = 0; e < 2; ++e) {
+            const int i = 2 * q + e;
+            const f2 D = e ? pack2(d.z, d.w) : pack2(d.x, d.y);
+            f2 c, s;
+            tc_sincos(e ? pack2(hi.z, hi.w) : pack2(hi.x, hi.y), e ? pack2(lo.z, lo.w) : pack2(lo.x, lo.y), D, H, F, c,
+                      s);
+            tc_split(c, ch[i], cl[i]);
+            tc_split(s, sh[i], sl[i]);
+            if (cross) {
+                const f2 x = fmul2(D, CX);
+                c1[i] = tc_half2(fmul2(c, x));
+                s1[i] = tc_half2(fmul2(s, x));
             }
         }
     }
@@ -233,21 +231,17 @@ __device__ __forceinline__ void make_b(unsigned char *b, uint32_t gs, const Chun
         return make_uint4(r[0] ^ flip, r[1] ^ flip, r[2] ^ flip, r[3] ^ flip);
     };
     constexpr uint32_t neg = 0x80008000u;
-#pragma unroll
-    for (int n = 0; n < NS; ++n) {
-        uint4 *o = reinterpret_cast<uint4 *>(b + ((gs + n) % kSlotsB) * Op<XR>::bytes + (uint32_t)w * Op<XR>::ks +
-                                             (uint32_t)lane * 16u);
-        o[0] = vec(ch[n], 0u);
-        o[XR] = o[6 * XR] = vec(sh[n], 0u);
-        o[2 * XR] = vec(cl[n], 0u);
-        o[3 * XR] = o[8 * XR] = vec(sl[n], 0u);
-        o[7 * XR] = vec(ch[n], neg);
-        o[9 * XR] = vec(cl[n], neg);
-        if (cross) {
-            o[4 * XR] = vec(s1[n], neg);
-            o[5 * XR] = o[10 * XR] = vec(c1[n], 0u);
-            o[11 * XR] = vec(s1[n], 0u);
-        }
+    uint4 *o = reinterpret_cast<uint4 *>(slot + (uint32_t)w * Op<XR>::ks + (uint32_t)lane * 16u);
+    o[0] = vec(ch, 0u);
+    o[XR] = o[6 * XR] = vec(sh, 0u);
+    o[2 * XR] = vec(cl, 0u);
+    o[3 * XR] = o[8 * XR] = vec(sl, 0u);
+    o[7 * XR] = vec(ch, neg);
+    o[9 * XR] = vec(cl, neg);
+    if (cross) {
+        o[4 * XR] = vec(s1, neg);
+        o[5 * XR] = o[10 * XR] = vec(c1, 0u);
+        o[11 * XR] = vec(s1, 0u);
     }
 }
 
@@ -336,9 +330,6 @@ __device__ __forceinline__ void column_role(const KernelArgs &a, Head *head, con
     volatile int *abort = &head->abort;
     const int warp = (threadIdx.x >> 5) & 3, x = threadIdx.x & 31;
     uint32_t gs = 0;
-    const auto wait_slot = [&](uint32_t g) {
-        if (g >= kSlotsB) tc_wait(&head->b_free[g % kSlotsB], ((g / kSlotsB) - 1) & 1, abort, a.status);
-    };
     for (uint32_t cn = 0;; ++cn) {
         const uint32_t buf = cn & 1;
         tc_wait(&head->c_full[buf], (cn >> 1) & 1, abort, a.status);
@@ -351,21 +342,12 @@ __device__ __forceinline__ void column_role(const KernelArgs &a, Head *head, con
         const float4 g0 = axis[x0 + 2 * (x >> 1)], g1 = axis[x0 + 2 * (x >> 1) + 1];
         const float h = x & 1 ? g0.y : g0.x, f = x & 1 ? g0.w : g0.z, cx = x & 1 ? g1.y : g1.x;
         const f2 H = pack2(h, h), F = pack2(f, f), CX = pack2(cx, cx);
-        int st = 0;
-        for (; st + 1 < stages; st += 2, gs += 2) {
-            wait_slot(gs);
-            wait_slot(gs + 1);
-            make_b<XR, 2>(smem + L.b, gs, data[buf], st * kStage + 8 * warp, H, F, CX, cross, x, warp);
+        for (int st = 0; st < stages; ++st, ++gs) {
+            const uint32_t slot = gs % kSlotsB;
+            if (gs >= kSlotsB) tc_wait(&head->b_free[slot], ((gs / kSlotsB) - 1) & 1, abort, a.status);
+            make_b<XR>(smem + L.b + slot * Op<XR>::bytes, data[buf], st * kStage + 8 * warp, H, F, CX, cross, x, warp);
             fence_proxy_async();
-            mbar_arrive(&head->b_full[gs % kSlotsB]);
-            mbar_arrive(&head->b_full[(gs + 1) % kSlotsB]);
-        }
-        if (st < stages) {
-            wait_slot(gs);
-            make_b<XR, 1>(smem + L.b, gs, data[buf], st * kStage + 8 * warp, H, F, CX, cross, x, warp);
-            fence_proxy_async();
-            mbar_arrive(&head->b_full[gs % kSlotsB]);
-            ++gs;
+            mbar_arrive(&head->b_full[slot]);
         }
         mbar_arrive(&head->c_free[buf]);
     }
@@ -429,7 +411,7 @@ __device__ __forceinline__ void factor_role(const KernelArgs &a, Head *head, con
         const float h = y & 1 ? g.y : g.x, f = y & 1 ? g.w : g.z;
         const f2 H = pack2(h, h), F = pack2(f, f);
         for (int st = (int)((gs ^ (uint32_t)wg) & 1u); st < stages; st += 2, ++uses) {
-#pragma unroll
+#pragma unroll 1
             for (int kb = 0; kb < 2; ++kb) {
                 const int slot = 2 * wg + kb;
                 uint32_t r[2][16];
@@ -476,7 +458,7 @@ __device__ __forceinline__ void sum_role(const KernelArgs &a, Head *head, const 
         const float4 g1 = axis[2 * (row >> 1) + 1];
         const float cy = row & 1 ? g1.y : g1.x;
         const f2 CY = pack2(cy, cy);
-#pragma unroll 2
+#pragma unroll 1
         for (int g = 0; g < 2 * XR / 16; ++g) {
             f2 vh[8], vl[8];
             const uint32_t col = tl + kColsD * buf + 16 * g;
@@ -517,15 +499,23 @@ __device__ __forceinline__ void sum_role(const KernelArgs &a, Head *head, const 
         const float4 *a1 = a.aterms + ((size_t)c.it.aterm * a.nr_stations + c.it.st1) * jones;
         const float4 *a2 = a.aterms + ((size_t)c.it.aterm * a.nr_stations + c.it.st2) * jones;
         const int gx = c.it.x0 + t;
-        if (t < sh.bs && gx < S) {
-#pragma unroll 2
-            for (int yy = 0; yy < 8; ++yy) {
-                const int gy = c.it.y0 + 8 * w + yy;
-                if (8 * w + yy >= sh.bs || gy >= S) break;
-                const int q = gy * S + gx;
+        const int rows = min(8, min(sh.bs, S - c.it.y0) - 8 * w);
+        if (t < sh.bs && gx < S && rows > 0) {
+            const int q0 = (c.it.y0 + 8 * w) * S + gx;
+            cf n1[4], n2[4]; // the next pixel's, on their way while this one is worked on
+            load_jones(a1 + 2 * q0, n1);
+            load_jones(a2 + 2 * q0, n2);
+#pragma unroll 1
+            for (int yy = 0; yy < rows; ++yy) {
+                const int gy = c.it.y0 + 8 * w + yy, q = q0 + yy * S, nq = q0 + min(yy + 1, rows - 1) * S;
                 cf j1[4], j2[4], px[4];
-                load_jones(a1 + 2 * q, j1);
-                load_jones(a2 + 2 * q, j2);
+#pragma unroll
+                for (int p = 0; p < 4; ++p) {
+                    j1[p] = n1[p];
+                    j2[p] = n2[p];
+                }
+                load_jones(a1 + 2 * nq, n1);
+                load_jones(a2 + 2 * nq, n2);
                 const float2 n = ntab[(gy < Sh ? gy : S - 1 - gy) * Sh + (gx < Sh ? gx : S - 1 - gx)];
                 const cf f = cscale(tc_pixel_factor(c.it.sg.g0h, c.it.sg.g0l, n), taper ? a.taper[q] : 1.f);
 #pragma unroll

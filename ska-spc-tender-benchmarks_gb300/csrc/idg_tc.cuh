@@ -135,8 +135,8 @@ __device__ __forceinline__ float tc_unord(unsigned u) {
 // (X + S/2 - G/2)/S modulo 2 as hi + lo: reduced as an integer over 2 S, the
 // remainder of the fp32 division recovered exactly.
 __device__ __forceinline__ void tc_offset(int X, int S, int G, float &hi, float &lo) {
-    int64_t r = (2 * (int64_t)X + S - G) % (4 * (int64_t)S);
-    const float n = (float)(int)r, q = (float)(2 * S);
+    const int r = (2 * (X % (2 * S)) + (S - G) % (4 * S)) % (4 * S);
+    const float n = (float)r, q = (float)(2 * S);
     hi = __fdiv_rn(n, q);
     lo = fmaf(-hi, q, n) / q;
 }
