@@ -7,6 +7,7 @@
 // gridding/src/degridding_benchmark.cu:205-318): allocate, copy in
 // `niterations` times, run `niterations` times, copy out, report
 // benchmark_result in microseconds and bytes per microsecond.
+#include <atomic>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -36,6 +37,9 @@ std::vector<DeviceWords> g_words;
 std::mutex g_shape_mutex;
 std::map<std::pair<int, int>, std::pair<int, int>> g_shapes;
 
+constexpr int kMaxDevices = 64;
+std::atomic<int> g_sms[kMaxDevices];
+
 int current_device() {
     int dev = 0;
     cudaGetDevice(&dev);
@@ -56,6 +60,31 @@ std::pair<int, int> &shapes_of(int S) {
     return it->second;
 }
 } // namespace
+
+LaunchDevice launch_device() {
+    LaunchDevice d;
+    d.error = cudaGetDevice(&d.device);
+    if (d.error != cudaSuccess) return d;
+    if (d.device < kMaxDevices) d.sms = g_sms[d.device].load(std::memory_order_relaxed);
+    if (d.sms == 0) {
+        d.error = cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, d.device);
+        if (d.error == cudaSuccess && d.device < kMaxDevices) g_sms[d.device].store(d.sms, std::memory_order_relaxed);
+    }
+    return d;
+}
+
+cudaError_t allow_dynamic_smem(const void *kernel, std::atomic<uint64_t> *done) {
+    const LaunchDevice d = launch_device();
+    if (d.error != cudaSuccess) return d.error;
+    const uint64_t bit = d.device < kMaxDevices ? uint64_t(1) << d.device : 0;
+    if (done->load(std::memory_order_acquire) & bit) return cudaSuccess;
+    int most = 0;
+    cudaError_t e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, d.device);
+    // 256 bytes are left for what the kernel declares statically
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most - 256);
+    if (e == cudaSuccess) done->fetch_or(bit, std::memory_order_release);
+    return e;
+}
 
 // Without the tensor cores: the mirror-quad gridder with 64 threads x 4 quads
 // (22; 24 with 512-visibility tiles for S = 32) where 64 threads cover whole

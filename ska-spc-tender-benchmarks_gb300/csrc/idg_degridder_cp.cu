@@ -1086,15 +1086,24 @@ cudaError_t launch_quad(const KernelArgs &a, cudaStream_t stream) {
     else
         kern = degridder_quad_kernel<NT, QB, MINB, CB, UNR, KSM, COL, RUN, PF, UNFIT>;
     const size_t smem = quad_layout(a.S, a.C, QB).total;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    int per_sm = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, NT, smem);
-    if (e != cudaSuccess) return e;
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    int64_t blocks = (int64_t)sms * (per_sm > 0 ? per_sm : 1);
+    int64_t blocks = 0;
+    cudaError_t e;
+    if constexpr (UNFIT) { // usually nothing to do: no queries
+        static std::atomic<uint64_t> allowed{0};
+        e = allow_dynamic_smem(reinterpret_cast<const void *>(kern), &allowed);
+        if (e != cudaSuccess) return e;
+        blocks = (int64_t)launch_device().sms * MINB;
+    } else {
+        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+        int per_sm = 0;
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, NT, smem);
+        if (e != cudaSuccess) return e;
+        int dev = 0, sms = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        blocks = (int64_t)sms * (per_sm > 0 ? per_sm : 1);
+    }
     if (a.share_den > 1) blocks = blocks / a.share_den > 0 ? blocks / a.share_den : 1;
     if (a.max_ctas > 0 && blocks > a.max_ctas) blocks = a.max_ctas;
     if (blocks > a.nr_subgrids) blocks = a.nr_subgrids;

@@ -622,12 +622,10 @@ cudaError_t launch(const KernelArgs &args, cudaStream_t stream) {
     KernelArgs a = args;
     a.tc = tc_const(a.S, a.image_size);
     const size_t smem = tc_layout<ROWS>(a.S, a.C).total;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    static std::atomic<uint64_t> allowed{0};
+    cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void *>(kern), &allowed);
     if (e != cudaSuccess) return e;
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    int64_t blocks = sms;
+    int64_t blocks = launch_device().sms;
     if (a.share_den > 1) blocks = blocks / a.share_den > 0 ? blocks / a.share_den : 1;
     if (a.max_ctas > 0 && blocks > a.max_ctas) blocks = a.max_ctas;
     // few subgrids: their tiles are shared out over the CTAs

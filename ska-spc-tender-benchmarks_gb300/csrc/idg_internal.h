@@ -1,12 +1,24 @@
 // idg_internal.h -- launch functions shared between the kernel files and the C ABI.
 #pragma once
 
+#include <atomic>
 #include <cstdint>
 #include <cuda_runtime.h>
 
 namespace idg {
 
 struct KernelArgs;
+
+// Launch-path queries, asked of the runtime once per device (a small call's host
+// time is a good part of it): the device's SM count, and the opt-in to as much
+// dynamic shared memory as a kernel can have.  `done` is a static of the caller,
+// one per kernel: bit d is set once device d has the opt-in.
+struct LaunchDevice {
+    int device = 0, sms = 0;
+    cudaError_t error = cudaSuccess;
+};
+LaunchDevice launch_device();
+cudaError_t allow_dynamic_smem(const void *kernel, std::atomic<uint64_t> *done);
 
 // IDG_VARIANT_PLAIN: one CTA per subgrid (idg_gridder.cu / idg_degridder.cu).
 // IDG_VARIANT_BATCHED: persistent packed-FP32x2 kernels (idg_*_fast.cu); need a.work_counter.
