@@ -23,8 +23,8 @@
 //    its S' into the other of two buffers while the tensor core works on the
 //    current one.
 // One CTA of 18 warps per SM: 448 columns of tensor memory, 147 KB of operands.
-// Measured on GB300, 4,416 subgrids of 128 x 16 visibilities at S = 32: 0.89 ms
-// (25 SM cycles per visibility beyond a fixed 7 us per subgrid and SM), against
+// Measured on GB300, 4,416 subgrids of 128 x 16 visibilities at S = 32: 0.87 ms
+// (24.6 SM cycles per visibility beyond a fixed 7 us per subgrid and SM), against
 // 5.27 ms for the mirror-quad kernel.  The products alone take 16 cycles per
 // visibility; the rest is the issue slots of the factor and result warps, which
 // share the SM's four schedulers.  28 subgrids of 64 x 16 in one call: 25 us
@@ -266,30 +266,29 @@ __device__ __forceinline__ void store_factors(uint32_t tm, const Shape &sh, cons
 // come first, the hi hi products last.  bh, bl, b1: descriptors of the group's
 // operands.
 template <int ROWS, int KJ, bool CROSS>
-__device__ __forceinline__ void issue_rows(uint32_t d, uint32_t am, uint32_t bh, uint32_t bl, uint32_t b1,
-                                           uint32_t lead) {
+__device__ __forceinline__ void issue_rows(uint32_t d, uint32_t am, uint32_t bh, uint32_t bl, uint32_t b1) {
     constexpr uint32_t id = umma_idesc_f16(128, 8 * ROWS), hi = umma_desc_hi(128);
     constexpr uint32_t w = 8 * KJ, dk = (2 * Op<ROWS>::ks) >> 4, off = (ROWS * 64) >> 4; // next 16 x; rows Si | -Sr
 #pragma unroll
     for (int j = 0; j < KJ; ++j) {
         const uint32_t c = am + 8u * (uint32_t)j, k = j * dk;
         if (j == 0)
-            umma_f16_ts<false, id, hi>(d, c, bl + k, lead);
+            umma_f16_ts<false, id, hi>(d, c, bl + k);
         else
-            umma_f16_ts<true, id, hi>(d, c, bl + k, lead);
-        umma_f16_ts<true, id, hi>(d, c + w, bh + k, lead);
-        umma_f16_ts<true, id, hi>(d, c + 2 * w, bl + k + off, lead);
-        umma_f16_ts<true, id, hi>(d, c + 3 * w, bh + k + off, lead);
+            umma_f16_ts<true, id, hi>(d, c, bl + k);
+        umma_f16_ts<true, id, hi>(d, c + w, bh + k);
+        umma_f16_ts<true, id, hi>(d, c + 2 * w, bl + k + off);
+        umma_f16_ts<true, id, hi>(d, c + 3 * w, bh + k + off);
         if (CROSS) {
-            umma_f16_ts<true, id, hi>(d, c + 4 * w, b1 + k + off, lead);
-            umma_f16_ts<true, (id | kUmmaNegateA), hi>(d, c + 5 * w, b1 + k, lead);
+            umma_f16_ts<true, id, hi>(d, c + 4 * w, b1 + k + off);
+            umma_f16_ts<true, (id | kUmmaNegateA), hi>(d, c + 5 * w, b1 + k);
         }
     }
 #pragma unroll
     for (int j = 0; j < KJ; ++j) {
         const uint32_t c = am + 8u * (uint32_t)j, k = j * dk;
-        umma_f16_ts<true, id, hi>(d, c, bh + k, lead);
-        umma_f16_ts<true, id, hi>(d, c + 2 * w, bh + k + off, lead);
+        umma_f16_ts<true, id, hi>(d, c, bh + k);
+        umma_f16_ts<true, id, hi>(d, c + 2 * w, bh + k + off);
     }
 }
 
@@ -511,50 +510,59 @@ __device__ __forceinline__ void result_role(const KernelArgs &a, Head *head, con
     }
 }
 
+// The tiles of one job.  n, r: tiles and row halves before them; b0: descriptor
+// of the operand set.
+template <int ROWS, int KJ, bool CROSS>
+__device__ __forceinline__ void issue_job(const KernelArgs &a, Head *head, const Shape &sh, uint32_t t0, uint32_t b0,
+                                          uint32_t n, int tiles, uint32_t lead) {
+    volatile int *abort = &head->abort;
+    const uint32_t group = Op<ROWS>::bytes >> 4, set = group * (uint32_t)sh.nq;
+    const uint32_t back = kAcc / (uint32_t)sh.nq; // tiles to an accumulator's last user
+#pragma unroll 1
+    for (int i = 0; i < tiles; ++i, ++n) {
+        const uint32_t w = n & 1, am = t0 + kColA + kColsA * w;
+        tc_wait(&head->a_full[w], (n >> 1) & 1, abort, a.status);
+#pragma unroll 1
+        for (uint32_t h = 0; h < (uint32_t)sh.nq; ++h) {
+            if (n >= back) tc_wait(&head->d_free[(n - back) & 1][h], ((n - back) >> 1) & 1, abort, a.status);
+            tmem_fence_after();
+            if (lead) {
+                const uint32_t bh = b0 + h * group;
+                issue_rows<ROWS, KJ, CROSS>(t0 + (sh.nq == 1 ? w : h) * 128u, am, bh, bh + set, bh + 2 * set);
+                umma_commit(&head->d_full[w][h]);
+                if (h + 1 == (uint32_t)sh.nq) umma_commit(&head->a_free[w]);
+            }
+            __syncwarp();
+        }
+    }
+}
+
 // One warp issues every product, tile by tile.
 template <int ROWS>
 __device__ __forceinline__ void issue_role(const KernelArgs &a, Head *head, const Shape &sh, const Layout &L,
                                            unsigned char *smem, uint32_t tm) {
     volatile int *abort = &head->abort;
-    const uint32_t lead = elect_lane();
-    uint32_t n = 0, r = 0, back_n = 0, back_h = 0; // tiles, row groups; the row group kAcc before
+    const uint32_t lead = elect_lane(), t0 = warp_uniform(tm);
+    uint32_t n = 0;
     for (uint32_t j = 0;; ++j) {
         const uint32_t buf = j & 1;
         tc_wait(&head->job_full[buf], (j >> 1) & 1, abort, a.status);
-        if (__any_sync(0xffffffffu, *abort) || head->job[buf].stop) break;
-        const uint32_t b0 = umma_desc_lo(smem_addr(smem + L.b + buf * L.bset), Op<ROWS>::ks);
-        const uint32_t group = Op<ROWS>::bytes >> 4, set = group * (uint32_t)sh.nq;
-        const int tiles = head->job[buf].t_end - head->job[buf].t_begin;
-        const bool cross = head->job[buf].sg.cross != 0;
-        for (int i = 0; i < tiles; ++i, ++n) {
-            const uint32_t w = n & 1, am = warp_uniform(tm + kColA + kColsA * w);
-            tc_wait(&head->a_full[w], (n >> 1) & 1, abort, a.status);
-            for (int h = 0; h < sh.nq; ++h, ++r) {
-                if (r >= kAcc) { // the accumulator's last user has read it
-                    tc_wait(&head->d_free[back_n & 1][back_h], (back_n >> 1) & 1, abort, a.status);
-                    if (++back_h == (uint32_t)sh.nq) {
-                        back_h = 0;
-                        ++back_n;
-                    }
-                }
-                __syncwarp();
-                tmem_fence_after();
-                const uint32_t d = warp_uniform(tm + (r % kAcc) * 128u), bh = warp_uniform(b0 + h * group);
-                const uint32_t bl = bh + set, b1 = bl + set;
-                if (sh.kx == 32) {
-                    if (cross)
-                        issue_rows<ROWS, 2, true>(d, am, bh, bl, b1, lead);
-                    else
-                        issue_rows<ROWS, 2, false>(d, am, bh, bl, b1, lead);
-                } else if (cross) {
-                    issue_rows<ROWS, 1, true>(d, am, bh, bl, b1, lead);
-                } else {
-                    issue_rows<ROWS, 1, false>(d, am, bh, bl, b1, lead);
-                }
-                if (lead) umma_commit(&head->d_full[w][h]);
-            }
-            if (lead) umma_commit(&head->a_free[w]);
+        __syncwarp();
+        if (__any_sync(0xffffffffu, *abort) || warp_uniform(head->job[buf].stop)) break;
+        const uint32_t b0 = warp_uniform(umma_desc_lo(smem_addr(smem + L.b + buf * L.bset), Op<ROWS>::ks));
+        const int tiles = (int)warp_uniform(head->job[buf].t_end - head->job[buf].t_begin);
+        const bool cross = warp_uniform(head->job[buf].sg.cross) != 0;
+        if (sh.kx == 32) {
+            if (cross)
+                issue_job<ROWS, 2, true>(a, head, sh, t0, b0, n, tiles, lead);
+            else
+                issue_job<ROWS, 2, false>(a, head, sh, t0, b0, n, tiles, lead);
+        } else if (cross) {
+            issue_job<ROWS, 1, true>(a, head, sh, t0, b0, n, tiles, lead);
+        } else {
+            issue_job<ROWS, 1, false>(a, head, sh, t0, b0, n, tiles, lead);
         }
+        n += (uint32_t)tiles;
         if (lead) umma_commit(&head->b_free[buf]);
         __syncwarp();
     }

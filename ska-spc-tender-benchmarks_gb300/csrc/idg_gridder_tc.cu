@@ -18,25 +18,29 @@
 //    products matter: a product costs its warp some 70 cycles to issue beside
 //    the other warps' work.  The first-order sum's factor cx(y) is a factor of
 //    the whole row and is applied when the sum is read.
-//  * Visibilities come in chunks of 128, each scaled by a power of two to the
+//  * Visibilities come in chunks of 256, each scaled by a power of two to the
 //    fp16 range, and go through in stages of 32.  The tensor core truncates its
 //    accumulator after every product, so the full-size and the small products
 //    have accumulators of their own and after each chunk their sum is added in
 //    fp32 to the block's sums in shared memory, while the next chunk fills the
 //    other buffer.
-//  * Roles: two factor warpgroups (A, alternate stages), one for the x-factors,
-//    one for the sums and the epilogue, two warps that bring in the chunks, one
-//    that issues the products, one that looks for the next subgrid.
-// One CTA of 20 warps per SM and all of its tensor memory.
-// Measured on GB300, 4,416 subgrids of 128 x 16 visibilities at S = 32: 1.38 ms
-// (43 SM cycles per visibility) against 5.02 ms for the mirror-quad kernel.  The
-// products take 16 of those cycles; shared memory (73 % of its wavefronts: every
-// factor warp reads every visibility, and with neighbouring lanes on different
-// visibilities a 16-byte read takes four) and the issue slots bound the rest.
-// The roles run five different loops on one SM, so these are kept small: with
-// the half stages unrolled and two stages of x-factors at a time, the same work
-// missed the instruction cache and took 1.47 ms.  28 subgrids of 64 x 16 in one
-// call: 42 us against 213 us.
+//  * Roles: four factor warpgroups that take stages in turn, both operands of
+//    one (an own half stage of A, an own stage of B each); a fifth for the sums
+//    and the epilogue; two warps that bring in the chunks, one that issues the
+//    products, one that looks for the next subgrid.
+// One CTA of 24 warps per SM and all of its tensor memory.
+// Measured on GB300, 4,416 subgrids of 128 x 16 visibilities at S = 32: 1.26 ms
+// (41 SM cycles per visibility) against 5.02 ms for the mirror-quad kernel.  The
+// products take 16 of those cycles.  The rest is the traffic of factors between
+// the roles: with the factors' arithmetic left out, or the loads, or the stores,
+// it stays near 30.  What helped: one warpgroup doing both operands of a stage
+// (one barrier less per stage, and the row and column factors of a warpgroup
+// overlap) in place of two for A and one for B, 1.31 against 1.37 ms, a fourth
+// such warpgroup, 1.26, and products issued by one thread inside one branch
+// instead of a predicate on each.  The roles run five different loops on one SM,
+// so these are kept small: with the half stages unrolled and two stages of
+// x-factors at a time, the same work missed the instruction cache (1.47 ms).
+// 28 subgrids of 64 x 16 in one call: 39 us against 213 us.
 #include "idg_tc.cuh"
 #include "idg_internal.h"
 
@@ -44,9 +48,9 @@ namespace idg {
 
 namespace {
 
-constexpr int kThreads = 4 * 128 + 4 * 32, kLoadThread = 4 * 128 + 64;
-constexpr int kChunk = 128, kStage = 32; // visibilities
-constexpr int kSlotsA = 4, kSlotsB = 4;  // half stages of A in tensor memory (two per factor warpgroup), stages of B
+constexpr int kWorkers = 4; // factor warpgroups
+constexpr int kThreads = (kWorkers + 1) * 128 + 4 * 32, kLoadThread = kThreads - 64;
+constexpr int kChunk = 256, kStage = 32; // visibilities
 constexpr uint32_t kColsD = 192, kColA = 384, kColsA = 32, kTmemCols = 512;
 constexpr uint32_t kAccStride = 128 * 16 + 16; // one group of four columns of the sums, padded
 
@@ -60,13 +64,12 @@ struct Item {
 
 struct Chunk {
     int stop, stages, first, last;
-    float inv;
+    float scale, inv;
     Item it;
 };
 
 struct Head {
-    uint64_t a_full[kSlotsA], a_free[kSlotsA];
-    uint64_t b_full[kSlotsB], b_free[kSlotsB];
+    uint64_t a_full[kWorkers], a_free[kWorkers];
     uint64_t c_full[2], c_free[2]; // chunks
     uint64_t d_full[2], d_free[2]; // accumulators
     uint64_t item_full, item_free, drain;
@@ -102,20 +105,18 @@ struct Op { // one stage of B
 };
 
 struct Layout {
-    size_t b, data, acc, axis, ntab, chan, total;
+    size_t b, data, acc, axis, ntab, total;
 };
 template <int XR>
-__host__ __device__ inline Layout tc_layout(int S, int C) {
+__host__ __device__ inline Layout tc_layout(int S) {
     const Shape s = tc_shape(S);
     Layout L;
     size_t off = (sizeof(Head) + 127) & ~size_t(127);
-    L.b = off;    off += (size_t)kSlotsB * Op<XR>::bytes;
+    L.b = off;    off += (size_t)kWorkers * Op<XR>::bytes;
     L.data = off; off += 2 * sizeof(ChunkData);
     L.acc = off;  off += (size_t)(2 * XR / 4) * kAccStride;
     L.axis = off; off += (size_t)(s.nb * s.bs / 2 + 16) * 32;
     L.ntab = off; off += (size_t)(S / 2) * (S / 2) * 8;
-    off = (off + 15) & ~size_t(15);
-    L.chan = off; off += (size_t)C * 16;
     L.total = off;
     return L;
 }
@@ -179,12 +180,11 @@ __device__ __forceinline__ void scout_role(const KernelArgs &a, Head *head, cons
 // The raw inputs of one visibility.
 struct Raw {
     float4 v0, v1;
-    float u, v, w;
-    float4 k;
+    float u, v, w, k;
 };
-__device__ __forceinline__ Raw load_raw(const KernelArgs &a, const float4 *chan, const Item &it, int chunk, int lane) {
+__device__ __forceinline__ Raw load_raw(const KernelArgs &a, const Item &it, int i) {
     Raw r;
-    const int i = chunk * kChunk + lane, j = min(i, it.nvis - 1);
+    const int j = min(i, it.nvis - 1);
     const int t = j / it.nc, c = it.c0 + j - t * it.nc;
     const float4 *src = a.vis + (((int64_t)it.row0 + t) * a.C + c) * 2;
     r.v0 = r.v1 = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -196,7 +196,7 @@ __device__ __forceinline__ Raw load_raw(const KernelArgs &a, const float4 *chan,
     r.u = p[0];
     r.v = p[1];
     r.w = p[2];
-    r.k = chan[c];
+    r.k = a.wavenumbers[c];
     return r;
 }
 
@@ -245,10 +245,9 @@ __device__ __forceinline__ void make_b(unsigned char *slot, const ChunkData &cd,
     }
 }
 
-// Chunks (two warps; a thread takes two visibilities).  The inputs of chunk
-// n + 1 are on their way while chunk n is made ready.
+// Chunks (two warps; a thread takes two visibilities at a time).  The next
+// inputs are on their way while these are made ready.
 __device__ __forceinline__ void load_role(const KernelArgs &a, Head *head, const Layout &L, unsigned char *smem) {
-    const float4 *chan = reinterpret_cast<const float4 *>(smem + L.chan);
     ChunkData *data = reinterpret_cast<ChunkData *>(smem + L.data);
     volatile int *abort = &head->abort;
     const int lane = (int)threadIdx.x - kLoadThread;
@@ -263,93 +262,58 @@ __device__ __forceinline__ void load_role(const KernelArgs &a, Head *head, const
         load_sync();
         mbar_arrive(&head->item_free);
         const int nchunks = stop ? 1 : (it.nvis + kChunk - 1) / kChunk;
-        Raw raw[2] = {};
+        Raw r0{}, r1{};
         if (!stop) {
-            raw[0] = load_raw(a, chan, it, 0, lane);
-            raw[1] = load_raw(a, chan, it, 0, lane + 64);
+            r0 = load_raw(a, it, lane);
+            r1 = load_raw(a, it, lane + 64);
         }
         for (int chunk = 0; chunk < nchunks; ++chunk, ++cn) {
             const uint32_t buf = cn & 1;
+            const int v0 = chunk * kChunk, stages = stop ? 0 : (min(it.nvis - v0, kChunk) + kStage - 1) / kStage;
+            if (cn >= 2) tc_wait(&head->c_free[buf], ((cn >> 1) - 1) & 1, abort, a.status);
+            ChunkData &cd = data[buf];
             unsigned m = 0u;
+#pragma unroll 1
+            for (int o = 0; o < stages * kStage; o += 64) {
+                const Raw r = r0;
+                const int n = o + lane;
+                r0 = r1;
+                if (v0 + o + 128 < it.nvis) r1 = load_raw(a, it, v0 + n + 128);
+                const float v[8] = {r.v0.x, r.v0.y, r.v0.z, r.v0.w, r.v1.x, r.v1.y, r.v1.z, r.v1.w};
 #pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const float v[8] = {raw[e].v0.x, raw[e].v0.y, raw[e].v0.z, raw[e].v0.w,
-                                    raw[e].v1.x, raw[e].v1.y, raw[e].v1.z, raw[e].v1.w};
-#pragma unroll
-                for (int i = 0; i < 8; ++i) m = max(m, __float_as_uint(fabsf(v[i])));
+                for (int i = 0; i < 8; ++i) {
+                    cd.v[i][n] = v[i];
+                    m = max(m, __float_as_uint(fabsf(v[i])));
+                }
+                const float ph = __fmul_rn(r.k, a.tc.d2h), pl = fmaf(r.k, a.tc.d2l, fmaf(r.k, a.tc.d2h, -ph));
+                const float qh = __fmul_rn(r.k, a.tc.i2h), ql = fmaf(r.k, a.tc.i2l, fmaf(r.k, a.tc.i2h, -qh));
+                float hi, lo;
+                tc_slope(ph, pl, r.u, it.sg.xh, it.sg.xl, hi, lo);
+                cd.ah[n] = hi;
+                cd.al[n] = kTwoPiF * lo;
+                tc_slope(ph, pl, r.v, it.sg.yh, it.sg.yl, hi, lo);
+                cd.bh[n] = hi;
+                cd.bl[n] = kTwoPiF * lo;
+                cd.d[n] = kTwoPiF * tc_delta(qh, ql, r.w, it.sg.mid);
             }
             m = __reduce_max_sync(0xffffffffu, m);
             if ((lane & 31) == 0) head->wmax[buf][lane >> 5] = m;
             load_sync();
-            float inv;
-            const float scale = tc_scale(max(head->wmax[buf][0], head->wmax[buf][1]), inv);
-            if (cn >= 2) tc_wait(&head->c_free[buf], ((cn >> 1) - 1) & 1, abort, a.status);
-            const int stages = stop ? 0 : (min(it.nvis - chunk * kChunk, kChunk) + kStage - 1) / kStage;
-            ChunkData &cd = data[buf];
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const Raw &r = raw[e];
-                const int n = lane + 64 * e;
-                const float v[8] = {r.v0.x, r.v0.y, r.v0.z, r.v0.w, r.v1.x, r.v1.y, r.v1.z, r.v1.w};
-#pragma unroll
-                for (int i = 0; i < 8; ++i) cd.v[i][n] = v[i] * scale;
-                float hi, lo;
-                tc_slope(r.k.x, r.k.y, r.u, it.sg.xh, it.sg.xl, hi, lo);
-                cd.ah[n] = hi;
-                cd.al[n] = kTwoPiF * lo;
-                tc_slope(r.k.x, r.k.y, r.v, it.sg.yh, it.sg.yl, hi, lo);
-                cd.bh[n] = hi;
-                cd.bl[n] = kTwoPiF * lo;
-                cd.d[n] = kTwoPiF * tc_delta(r.k.z, r.k.w, r.w, it.sg.mid);
-            }
             if (lane == 0) {
                 Chunk &c = head->chunk[buf];
+                float inv;
+                c.scale = tc_scale(max(head->wmax[buf][0], head->wmax[buf][1]), inv);
+                // the accumulator is truncated after each of 4 products per stage: see kTcTruncation
+                c.inv = inv * (1.f + kTcTruncationPerStage * (float)stages);
                 c.stop = stop;
                 c.stages = stages;
                 c.first = chunk == 0;
                 c.last = chunk == nchunks - 1;
-                // the accumulator is truncated after each of 4 products per stage: see kTcTruncation
-                c.inv = inv * (1.f + kTcTruncationPerStage * (float)stages);
                 c.it = it;
             }
             mbar_arrive(&head->c_full[buf]);
-            if (chunk + 1 < nchunks) {
-                raw[0] = load_raw(a, chan, it, chunk + 1, lane);
-                raw[1] = load_raw(a, chan, it, chunk + 1, lane + 64);
-            }
         }
         if (stop) return;
-    }
-}
-
-// x-factors (one warpgroup).
-template <int XR>
-__device__ __forceinline__ void column_role(const KernelArgs &a, Head *head, const Layout &L, unsigned char *smem) {
-    const float4 *axis = reinterpret_cast<const float4 *>(smem + L.axis);
-    const ChunkData *data = reinterpret_cast<const ChunkData *>(smem + L.data);
-    volatile int *abort = &head->abort;
-    const int warp = (threadIdx.x >> 5) & 3, x = threadIdx.x & 31;
-    uint32_t gs = 0;
-    for (uint32_t cn = 0;; ++cn) {
-        const uint32_t buf = cn & 1;
-        tc_wait(&head->c_full[buf], (cn >> 1) & 1, abort, a.status);
-        __syncwarp();
-        if (__any_sync(0xffffffffu, *abort)) return;
-        const Chunk &c = head->chunk[buf];
-        if (c.stop) return;
-        const int stages = c.stages, x0 = c.it.x0;
-        const bool cross = c.it.sg.cross != 0;
-        const float4 g0 = axis[x0 + 2 * (x >> 1)], g1 = axis[x0 + 2 * (x >> 1) + 1];
-        const float h = x & 1 ? g0.y : g0.x, f = x & 1 ? g0.w : g0.z, cx = x & 1 ? g1.y : g1.x;
-        const f2 H = pack2(h, h), F = pack2(f, f), CX = pack2(cx, cx);
-        for (int st = 0; st < stages; ++st, ++gs) {
-            const uint32_t slot = gs % kSlotsB;
-            if (gs >= kSlotsB) tc_wait(&head->b_free[slot], ((gs / kSlotsB) - 1) & 1, abort, a.status);
-            make_b<XR>(smem + L.b + slot * Op<XR>::bytes, data[buf], st * kStage + 8 * warp, H, F, CX, cross, x, warp);
-            fence_proxy_async();
-            mbar_arrive(&head->b_full[slot]);
-        }
-        mbar_arrive(&head->c_free[buf]);
     }
 }
 
@@ -366,15 +330,19 @@ __device__ __forceinline__ void tmem_st_16x256_x4(uint32_t addr, const uint32_t 
 // of visibilities; r[0] for polarisations 0, 1 (lanes 0 .. 15 of the warp's
 // quarter), r[1] for 2, 3 (16 .. 31).  Columns: Re hi | Re lo | Im hi | Im lo,
 // eight each.
-__device__ __forceinline__ void make_a(uint32_t (&r)[2][16], const ChunkData &cd, int v0, f2 H, f2 F) {
+__device__ __forceinline__ void make_a(uint32_t (&r)[2][16], const ChunkData &cd, int v0, f2 H, f2 F, f2 SC) {
     const float4 hi = *reinterpret_cast<const float4 *>(&cd.bh[v0]);
     const float4 lo = *reinterpret_cast<const float4 *>(&cd.bl[v0]);
     const float4 d = *reinterpret_cast<const float4 *>(&cd.d[v0]);
     f2 c[2], s[2], n[2];
     tc_sincos(pack2(hi.x, hi.y), pack2(lo.x, lo.y), pack2(d.x, d.y), H, F, c[0], s[0]);
     tc_sincos(pack2(hi.z, hi.w), pack2(lo.z, lo.w), pack2(d.z, d.w), H, F, c[1], s[1]);
-    n[0] = s[0] ^ 0x8000000080000000ull;
-    n[1] = s[1] ^ 0x8000000080000000ull;
+#pragma unroll
+    for (int b = 0; b < 2; ++b) { // the chunk's power of two goes in here
+        c[b] = fmul2(c[b], SC);
+        s[b] = fmul2(s[b], SC);
+        n[b] = s[b] ^ 0x8000000080000000ull;
+    }
 #pragma unroll
     for (int p = 0; p < 4; ++p) {
         const float4 vr = *reinterpret_cast<const float4 *>(&cd.v[2 * p][v0]);
@@ -391,14 +359,15 @@ __device__ __forceinline__ void make_a(uint32_t (&r)[2][16], const ChunkData &cd
     }
 }
 
-// Factor warpgroups: A of alternate stages.
+// Factor warpgroups: both factors of every kWorkers-th stage.
+template <int XR>
 __device__ __forceinline__ void factor_role(const KernelArgs &a, Head *head, const Layout &L, unsigned char *smem,
                                             uint32_t tl) {
     const float4 *axis = reinterpret_cast<const float4 *>(smem + L.axis);
     const ChunkData *data = reinterpret_cast<const ChunkData *>(smem + L.data);
     volatile int *abort = &head->abort;
-    const int wg = threadIdx.x >> 7, t = threadIdx.x & 31, row = 8 * ((threadIdx.x >> 5) & 3) + (t >> 2);
-    uint32_t gs = 0, uses = 0;
+    const int wg = threadIdx.x >> 7, warp = (threadIdx.x >> 5) & 3, t = threadIdx.x & 31, row = 8 * warp + (t >> 2);
+    uint32_t turn = (uint32_t)wg, uses = 0; // stages until this warpgroup's next one; those it has done
     for (uint32_t cn = 0;; ++cn) {
         const uint32_t buf = cn & 1;
         tc_wait(&head->c_full[buf], (cn >> 1) & 1, abort, a.status);
@@ -406,27 +375,37 @@ __device__ __forceinline__ void factor_role(const KernelArgs &a, Head *head, con
         if (__any_sync(0xffffffffu, *abort)) return;
         const Chunk &c = head->chunk[buf];
         if (c.stop) return;
-        const int stages = c.stages, y = c.it.y0 + row;
-        const float4 g = axis[2 * (y >> 1)];
-        const float h = y & 1 ? g.y : g.x, f = y & 1 ? g.w : g.z;
-        const f2 H = pack2(h, h), F = pack2(f, f);
-        for (int st = (int)((gs ^ (uint32_t)wg) & 1u); st < stages; st += 2, ++uses) {
+        const uint32_t stages = (uint32_t)c.stages;
+        const int y = c.it.y0 + row, x0 = c.it.x0;
+        const bool cross = c.it.sg.cross != 0;
+        const float scale = c.scale;
+        for (; turn < stages; turn += kWorkers, ++uses) {
+            const int v0 = (int)turn * kStage;
+            const float4 g = axis[2 * (y >> 1)];
+            const float h = y & 1 ? g.y : g.x, f = y & 1 ? g.w : g.z;
 #pragma unroll 1
-            for (int kb = 0; kb < 2; ++kb) {
-                const int slot = 2 * wg + kb;
+            for (uint32_t kb = 0; kb < 2; ++kb) {
                 uint32_t r[2][16];
-                make_a(r, data[buf], st * kStage + 16 * kb + 4 * (t & 3), H, F);
-                if (uses > 0) tc_wait(&head->a_free[slot], (uses - 1) & 1, abort, a.status);
+                make_a(r, data[buf], v0 + 16 * (int)kb + 4 * (t & 3), pack2(h, h), pack2(f, f), pack2(scale, scale));
+                // the products of this warpgroup's previous half stage, and all before it, have read A and B
+                if (uses > 0 || kb > 0) tc_wait(&head->a_free[wg], (kb + 1) & 1, abort, a.status);
                 __syncwarp();
                 tmem_fence_after();
-                tmem_st_16x256_x4(tl + kColA + kColsA * slot, r[0]);
-                tmem_st_16x256_x4(tl + kColA + kColsA * slot + (16u << 16), r[1]);
+                tmem_st_16x256_x4(tl + kColA + kColsA * wg, r[0]);
+                tmem_st_16x256_x4(tl + kColA + kColsA * wg + (16u << 16), r[1]);
+                if (kb == 0) {
+                    const float4 g0 = axis[x0 + 2 * (t >> 1)], g1 = axis[x0 + 2 * (t >> 1) + 1];
+                    const float hx = t & 1 ? g0.y : g0.x, fx = t & 1 ? g0.w : g0.z, cx = t & 1 ? g1.y : g1.x;
+                    make_b<XR>(smem + L.b + wg * Op<XR>::bytes, data[buf], v0 + 8 * warp, pack2(hx, hx), pack2(fx, fx),
+                               pack2(cx, cx), cross, t, warp);
+                    fence_proxy_async();
+                }
                 tmem_wait_st();
                 tmem_fence_before();
-                mbar_arrive(&head->a_full[slot]);
+                mbar_arrive(&head->a_full[wg]);
             }
         }
-        gs += (uint32_t)stages;
+        turn -= stages;
         mbar_arrive(&head->c_free[buf]);
     }
 }
@@ -537,15 +516,45 @@ __device__ __forceinline__ void sum_role(const KernelArgs &a, Head *head, const 
     }
 }
 
-// The products of 16 visibilities.
+// The products of 16 visibilities (one thread).
 template <int XR, bool CROSS>
-__device__ __forceinline__ void issue_step(uint32_t d, uint32_t c, uint32_t k, uint32_t acc, uint32_t lead) {
+__device__ __forceinline__ void issue_step(uint32_t d, uint32_t c, uint32_t k, uint32_t acc) {
     constexpr uint32_t hi = umma_desc_hi(128);
     constexpr uint32_t id = umma_idesc_f16(128, (CROSS ? 6 : 4) * XR), idl = umma_idesc_f16(128, 2 * XR);
-    umma_f16_ts_if<id, hi>(d, c, k, acc, lead);
-    umma_f16_ts<true, (id | kUmmaNegateA), hi>(d, c + 16, k + 6 * XR, lead);
-    umma_f16_ts<true, idl, hi>(d + 2 * XR, c + 8, k, lead);
-    umma_f16_ts<true, (idl | kUmmaNegateA), hi>(d + 2 * XR, c + 24, k + 6 * XR, lead);
+    umma_f16_ts_if<id, hi>(d, c, k, acc);
+    umma_f16_ts<true, (id | kUmmaNegateA), hi>(d, c + 16, k + 6 * XR);
+    umma_f16_ts<true, idl, hi>(d + 2 * XR, c + 8, k);
+    umma_f16_ts<true, (idl | kUmmaNegateA), hi>(d + 2 * XR, c + 24, k + 6 * XR);
+}
+
+// The stages of one chunk: the warpgroups' first half stages, then their second
+// ones, so that each is formed while the others' are multiplied.  gs: stages
+// before this chunk; c0, b0: the warpgroups' first A columns and B descriptor.
+template <int XR, bool CROSS>
+__device__ __forceinline__ void issue_chunk(const KernelArgs &a, Head *head, uint32_t d, uint32_t c0, uint32_t b0,
+                                            uint32_t gs, int stages, uint32_t lead) {
+    volatile int *abort = &head->abort;
+    uint32_t acc = 0;
+    for (int st = 0; st < stages; st += kWorkers, gs += kWorkers) {
+        const uint32_t n = (uint32_t)min(kWorkers, stages - st);
+#pragma unroll 1
+        for (uint32_t kb = 0; kb < 2; ++kb) {
+            uint32_t w = gs % kWorkers;
+#pragma unroll 1
+            for (uint32_t i = 0; i < n; ++i) {
+                tc_wait(&head->a_full[w], kb, abort, a.status); // with kb = 0, B too
+                tmem_fence_after();
+                if (lead) {
+                    issue_step<XR, CROSS>(d, c0 + kColsA * w,
+                                          b0 + (Op<XR>::bytes >> 4) * w + ((2 * Op<XR>::ks) >> 4) * kb, acc);
+                    umma_commit(&head->a_free[w]);
+                }
+                __syncwarp();
+                acc = 1;
+                w = w + 1 == kWorkers ? 0 : w + 1;
+            }
+        }
+    }
 }
 
 template <int XR>
@@ -553,39 +562,24 @@ __device__ __forceinline__ void issue_role(const KernelArgs &a, Head *head, cons
                                            uint32_t tm) {
     volatile int *abort = &head->abort;
     const uint32_t lead = elect_lane();
-    const uint32_t b0 = umma_desc_lo(smem_addr(smem + L.b), Op<XR>::ks);
+    const uint32_t t0 = warp_uniform(tm), b0 = warp_uniform(umma_desc_lo(smem_addr(smem + L.b), Op<XR>::ks));
     uint32_t gs = 0;
     for (uint32_t cn = 0;; ++cn) {
         const uint32_t buf = cn & 1;
         tc_wait(&head->c_full[buf], (cn >> 1) & 1, abort, a.status);
         __syncwarp();
         if (__any_sync(0xffffffffu, *abort)) break;
-        const int stop = head->chunk[buf].stop, stages = head->chunk[buf].stages;
-        const bool cross = head->chunk[buf].it.sg.cross != 0;
-        __syncwarp();
+        const bool stop = warp_uniform(head->chunk[buf].stop) != 0, cross = warp_uniform(head->chunk[buf].it.sg.cross) != 0;
+        const int stages = (int)warp_uniform(head->chunk[buf].stages);
         mbar_arrive(&head->c_free[buf]);
         if (stop) break;
         if (cn >= 2) tc_wait(&head->d_free[buf], ((cn >> 1) - 1) & 1, abort, a.status);
-        const uint32_t d = warp_uniform(tm + kColsD * buf);
-        for (int st = 0; st < stages; ++st, ++gs) {
-            const uint32_t sb = gs % kSlotsB, b = warp_uniform(b0 + sb * (Op<XR>::bytes >> 4));
-            tc_wait(&head->b_full[sb], (gs / kSlotsB) & 1, abort, a.status);
-#pragma unroll
-            for (uint32_t kb = 0; kb < 2; ++kb) {
-                const uint32_t sa = 2 * (gs & 1) + kb, c = warp_uniform(tm + kColA + kColsA * sa);
-                tc_wait(&head->a_full[sa], (gs >> 1) & 1, abort, a.status);
-                __syncwarp();
-                tmem_fence_after();
-                const uint32_t k = b + kb * ((2 * Op<XR>::ks) >> 4), acc = st > 0 || kb > 0;
-                if (cross)
-                    issue_step<XR, true>(d, c, k, acc, lead);
-                else
-                    issue_step<XR, false>(d, c, k, acc, lead);
-                if (lead) umma_commit(&head->a_free[sa]);
-            }
-            if (lead) umma_commit(&head->b_free[sb]);
-            __syncwarp();
-        }
+        __syncwarp();
+        if (cross)
+            issue_chunk<XR, true>(a, head, t0 + kColsD * buf, t0 + kColA, b0, gs, stages, lead);
+        else
+            issue_chunk<XR, false>(a, head, t0 + kColsD * buf, t0 + kColA, b0, gs, stages, lead);
+        gs += (uint32_t)stages;
         if (lead) umma_commit(&head->d_full[buf]);
         __syncwarp();
     }
@@ -600,26 +594,23 @@ template <int XR>
 __global__ void __launch_bounds__(kThreads, 1) gridder_tc_kernel(KernelArgs a) {
     extern __shared__ __align__(128) unsigned char smem[];
     const Shape sh = tc_shape(a.S);
-    const Layout L = tc_layout<XR>(a.S, a.C);
+    const Layout L = tc_layout<XR>(a.S);
     Head *head = reinterpret_cast<Head *>(smem);
     const int tid = threadIdx.x, warp = tid >> 5;
 
-    if (warp == 16) {
+    constexpr int kSum = 4 * kWorkers, kIssue = kSum + 4; // first warps of the roles behind the factor warpgroups
+    if (warp == kIssue) {
         tmem_alloc(&head->tmem, kTmemCols);
         tmem_relinquish();
     }
     if (tid == 0) {
-        for (int i = 0; i < kSlotsA; ++i) {
+        for (int i = 0; i < kWorkers; ++i) {
             mbar_init(&head->a_full[i], 128);
             mbar_init(&head->a_free[i], 1);
         }
-        for (int i = 0; i < kSlotsB; ++i) {
-            mbar_init(&head->b_full[i], 128);
-            mbar_init(&head->b_free[i], 1);
-        }
         for (int i = 0; i < 2; ++i) {
             mbar_init(&head->c_full[i], 64);
-            mbar_init(&head->c_free[i], 256 + 128 + 128 + 32);
+            mbar_init(&head->c_free[i], 128 * kWorkers + 128 + 32);
             mbar_init(&head->d_full[i], 1);
             mbar_init(&head->d_free[i], 128);
         }
@@ -631,27 +622,24 @@ __global__ void __launch_bounds__(kThreads, 1) gridder_tc_kernel(KernelArgs a) {
     }
     tc_axis_table(a, reinterpret_cast<float4 *>(smem + L.axis), sh.nb * sh.bs / 2 + 16, tid, kThreads);
     tc_n_table(a, reinterpret_cast<float2 *>(smem + L.ntab), tid, kThreads);
-    tc_channel_table(a, reinterpret_cast<float4 *>(smem + L.chan), tid, kThreads);
     tmem_fence_before();
     __syncthreads();
     tmem_fence_after();
     const uint32_t tm = head->tmem;
     const uint32_t tl = tm + ((uint32_t)(warp & 3) << 21); // this warp's lane quarter
 
-    if (warp < 8)
-        factor_role(a, head, L, smem, tl);
-    else if (warp < 12)
-        column_role<XR>(a, head, L, smem);
-    else if (warp < 16)
+    if (warp < kSum)
+        factor_role<XR>(a, head, L, smem, tl);
+    else if (warp < kIssue)
         sum_role<XR>(a, head, L, smem, tl, sh);
-    else if (warp == 16)
+    else if (warp == kIssue)
         issue_role<XR>(a, head, L, smem, tm);
-    else if (warp == 17)
+    else if (warp == kIssue + 1)
         scout_role(a, head, sh);
     else
         load_role(a, head, L, smem);
     __syncthreads();
-    if (warp == 16) tmem_free(tm, kTmemCols);
+    if (warp == kIssue) tmem_free(tm, kTmemCols);
 }
 
 template <int XR>
@@ -663,7 +651,7 @@ cudaError_t launch(const KernelArgs &args, cudaStream_t stream, bool load_only) 
     }
     KernelArgs a = args;
     a.tc = tc_const(a.S, a.image_size);
-    const size_t smem = tc_layout<XR>(a.S, a.C).total;
+    const size_t smem = tc_layout<XR>(a.S).total;
     static std::atomic<uint64_t> allowed{0};
     cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void *>(kern), &allowed);
     if (e != cudaSuccess) return e;

@@ -47,27 +47,25 @@ __device__ __forceinline__ uint32_t umma_desc_lo(uint32_t addr, uint32_t k_strid
 }
 // A value that is the same in every lane, for the compiler to see as such.
 __device__ __forceinline__ uint32_t warp_uniform(uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); }
-// D[tmem] (+)= A[tmem] B[smem].  A whole converged warp calls it and the lane
-// with `lead` issues: with warp-uniform operands and constant descriptor parts
-// a product takes a few cycles to issue, where a loop run by one thread on
-// run-time descriptors took 126 (the tensor core needs 32 for N = 64).
+// D[tmem] (+)= A[tmem] B[smem]; one thread issues.  Operands that are uniform
+// over its warp and constant descriptor parts keep this to a few instructions; a
+// loop on run-time descriptors took 126 cycles per product (the tensor core
+// needs 32 for N = 64).
 template <bool ACC, uint32_t IDESC, uint32_t DESC_HI>
-__device__ __forceinline__ void umma_f16_ts(uint32_t d, uint32_t a, uint32_t b_lo, uint32_t lead) {
+__device__ __forceinline__ void umma_f16_ts(uint32_t d, uint32_t a, uint32_t b_lo) {
     asm volatile(
-        "{\n .reg .pred p, q;\n .reg .b64 b;\n setp.ne.u32 q, %3, 0;\n setp.ne.u32 p, %4, 0;\n"
-        " mov.b64 b, {%2, %6};\n"
-        " @q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %5, p;\n}\n" ::"r"(d),
-        "r"(a), "r"(b_lo), "r"(lead), "n"(ACC ? 1 : 0), "r"(IDESC), "r"(DESC_HI)
+        "{\n .reg .pred p;\n .reg .b64 b;\n setp.ne.u32 p, %3, 0;\n mov.b64 b, {%2, %5};\n"
+        " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %4, p;\n}\n" ::"r"(d),
+        "r"(a), "r"(b_lo), "n"(ACC ? 1 : 0), "r"(IDESC), "r"(DESC_HI)
         : "memory");
 }
 // The same with the choice at run time.
 template <uint32_t IDESC, uint32_t DESC_HI>
-__device__ __forceinline__ void umma_f16_ts_if(uint32_t d, uint32_t a, uint32_t b_lo, uint32_t acc, uint32_t lead) {
+__device__ __forceinline__ void umma_f16_ts_if(uint32_t d, uint32_t a, uint32_t b_lo, uint32_t acc) {
     asm volatile(
-        "{\n .reg .pred p, q;\n .reg .b64 b;\n setp.ne.u32 q, %3, 0;\n setp.ne.u32 p, %4, 0;\n"
-        " mov.b64 b, {%2, %6};\n"
-        " @q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %5, p;\n}\n" ::"r"(d),
-        "r"(a), "r"(b_lo), "r"(lead), "r"(acc), "r"(IDESC), "r"(DESC_HI)
+        "{\n .reg .pred p;\n .reg .b64 b;\n setp.ne.u32 p, %3, 0;\n mov.b64 b, {%2, %5};\n"
+        " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %4, p;\n}\n" ::"r"(d),
+        "r"(a), "r"(b_lo), "r"(acc), "r"(IDESC), "r"(DESC_HI)
         : "memory");
 }
 // The mbarrier completes a phase when every MMA issued so far by this thread has finished.
