@@ -119,6 +119,13 @@ __device__ __forceinline__ void fft_1d(cf *x, const float2 *tw) {
     }
 }
 
+// v conj(cy cx), the factor before the backward transform, with its roundings
+// spelled out: the fused pass gives the bits of the splitter followed by this.
+__device__ __forceinline__ float2 before_backward(float2 v, float2 cy, float2 cx) {
+    const float re = fmaf(cy.x, cx.x, -__fmul_rn(cy.y, cx.y)), im = fmaf(cy.x, cx.y, __fmul_rn(cy.y, cx.x));
+    return make_float2(fmaf(v.x, re, __fmul_rn(v.y, im)), fmaf(v.y, re, -__fmul_rn(v.x, im)));
+}
+
 template <int S>
 struct FftShape {
     static constexpr int planes = S >= 64 ? 1 : 128 / S; // <= 48 KiB of static shared memory
@@ -208,10 +215,7 @@ __global__ void __launch_bounds__(FftShape<S>::threads) subgrid_fft_kernel(float
                         const float f = (((xx + y) & 1) ? -1.f : 1.f) * (taper ? __ldg(taper + q) : 1.f);
                         w = make_float2(w.x * f, w.y * f);
                     } else {
-                        const float2 cy = post[y], cx = post[xx];
-                        const cf c = cconj(cmul({cy.x, cy.y}, {cx.x, cx.y}));
-                        const cf rr = cmul({w.x, w.y}, c);
-                        w = make_float2(rr.re, rr.im);
+                        w = before_backward(w, post[y], post[xx]);
                     }
                     buf[p2][y][xx] = w;
                 }
@@ -222,28 +226,32 @@ __global__ void __launch_bounds__(FftShape<S>::threads) subgrid_fft_kernel(float
 #pragma unroll
             for (int i = 0; i < S; ++i) x[i] = {buf[pl][r][i].x, buf[pl][r][i].y};
         }
-    } else if (pl < nplanes) {
-        // The split pass gathers grid rows: thread (pl, r) reads row r of its
-        // plane's footprint straight into registers and pre-multiplies it.
-        const PlaneSrc ps = src_of[pl];
-        const int step = ps.mirror ? -1 : 1;
-        const int gy = ps.y0 + step * r;
-        const bool row_ok = ps.base >= 0 && gy >= 0 && gy < sa.G;
-        const float2 *grow = sa.grid + (row_ok ? ps.base + (int64_t)gy * sa.G : 0);
-        // all of the row's loads first (independent, in flight together),
-        // then the pre-multiplication
+    } else {
+        // The split pass gathers the footprints' rows: thread (pl, r) reads column
+        // r of its plane, so that neighbouring threads read neighbouring cells, all
+        // loads in flight together, and leaves it pre-multiplied in shared memory.
+        // (With a row per thread every load touched 32 lines: 8,128 subgrids of
+        // 32^2 took 165 us, this way 97, grid and subgrids 59 us at the copy rate.)
+        if (pl < nplanes) {
+            const PlaneSrc ps = src_of[pl];
+            const int step = ps.mirror ? -1 : 1, gx = ps.x0 + step * r;
+            const bool col_ok = ps.base >= 0 && (unsigned)gx < (unsigned)sa.G;
+            const int64_t down = (int64_t)step * sa.G;
+            const float2 *col = sa.grid + (col_ok ? ps.base + (int64_t)ps.y0 * sa.G + gx : 0);
 #pragma unroll
-        for (int i = 0; i < S; ++i) {
-            const int gx = ps.x0 + step * i;
-            float2 v = make_float2(0.f, 0.f);
-            if (row_ok && gx >= 0 && gx < sa.G) v = __ldg(grow + gx);
-            x[i] = {v.x, ps.mirror ? -v.y : v.y};
+            for (int i = 0; i < S; ++i) {
+                float2 v = make_float2(0.f, 0.f);
+                if (col_ok && (unsigned)(ps.y0 + step * i) < (unsigned)sa.G) v = __ldg(col + i * down);
+                x[i] = {v.x, ps.mirror ? -v.y : v.y};
+            }
+            const float2 cx = post[r];
+#pragma unroll
+            for (int i = 0; i < S; ++i) buf[pl][i][r] = before_backward({x[i].re, x[i].im}, post[i], cx);
         }
+        __syncthreads();
+        if (pl < nplanes) {
 #pragma unroll
-        for (int i = 0; i < S; ++i) {
-            const float2 cy = post[r], cx = post[i];
-            const cf c = cconj(cmul({cy.x, cy.y}, {cx.x, cx.y}));
-            x[i] = cmul(x[i], c);
+            for (int i = 0; i < S; ++i) x[i] = {buf[pl][r][i].x, buf[pl][r][i].y};
         }
     }
     if (pl < nplanes) {
