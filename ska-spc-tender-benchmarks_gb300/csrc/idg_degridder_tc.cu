@@ -41,6 +41,7 @@ namespace {
 constexpr int kGen = 256;                 // factor threads (two warpgroups)
 constexpr int kThreads = 2 * kGen + 64;   // + two result warpgroups, the issuing and the scouting warp
 constexpr int kTile = 128;                // visibilities per tile
+constexpr int kGroup = 4, kSegTiles = 16; // subgrids sharing their long ones, least tiles of a segment
 constexpr int kAcc = 2;                   // accumulators of 128 columns: (re | im) x ROWS x 4 polarisations
 constexpr uint32_t kColA = 256, kColsA = 96, kTmemCols = 512;
 
@@ -292,30 +293,73 @@ __device__ __forceinline__ void issue_rows(uint32_t d, uint32_t am, uint32_t bh,
     }
 }
 
-// The scouting warp: takes subgrids from the work counter, leaves out what the
+// The scouting warp: takes work from the counter, leaves out what the
 // expansion does not hold for, and asks L2 for the pixels and A-terms of the
 // others.
+//  * nseg > 0 (fewer subgrids than CTAs): a claim is one of nseg equal segments
+//    of a subgrid's tiles.
+//  * nseg = 0: a claim is one of kGroup subgrids of a group, shared like this: a
+//    subgrid of 2 kSegTiles tiles or more is cut into up to kGroup segments
+//    (as many as the group has members), and claim q of a group takes segment
+//    q - j modulo the members of its subgrid j.
+//    So there are as many claims as subgrids, a short subgrid (one segment) is
+//    one claim, and a long one is spread over its neighbours' claims: one of
+//    16,384 visibilities at S = 48 held its SM for 0.75 ms at the end of the
+//    call.  Degridding steps, whole and shared: 1,500 subgrids of 128 to 16,384
+//    visibilities at S = 48 2.01 and 1.59 ms, 600 at S = 32 408 and 271 us, 1,500
+//    at S = 24 539 and 446; for 4,416 even ones the look at the neighbours costs
+//    5 of 880 us, of one tile each 6 of 228.  Claims for every segment, the empty
+//    ones too, made that last call 299 us.
 __device__ __forceinline__ void scout_role(const KernelArgs &a, int nseg, Head *head) {
     volatile int *abort = &head->abort;
     const int lane = threadIdx.x & 31;
     const size_t jones = (size_t)a.S * a.S * 2; // float4 per matrix plane
-    for (uint32_t k = 0;;) {
+    uint32_t k = 0;
+    auto publish = [&](const Item &it) {
+        if (k > 0) tc_wait(&head->item_free, (k - 1) & 1, abort, a.status);
+        __syncwarp();
+        if (lane == 0) {
+            head->item = it;
+            mbar_arrive(&head->item_full);
+        }
+        ++k;
+    };
+    for (;;) {
         int item = 0;
         if (lane == 0) item = *abort ? INT32_MAX : atomicAdd(a.work_counter, 1);
         item = __shfl_sync(0xffffffffu, item, 0);
         Item it{};
-        it.stop = item >= a.nr_subgrids * nseg;
-        if (!it.stop) {
-            const int idx = item / nseg, seg = item - idx * nseg;
-            const int s = a.work_list ? a.work_list[idx] : idx;
-            const SubgridInfo si = load_subgrid(a, s);
+        if (item >= a.nr_subgrids * (nseg > 0 ? nseg : 1)) {
+            it.stop = 1;
+            publish(it);
+            return;
+        }
+        // the claim's own subgrid, and on lane j how subgrid j of its group is cut
+        const int q = nseg > 0 ? 0 : item % kGroup, first = nseg > 0 ? item / nseg : item - q;
+        auto subgrid = [&](int j) { return a.work_list ? a.work_list[first + j] : first + j; };
+        SubgridInfo si = load_subgrid(a, subgrid(q));
+        const int members = nseg > 0 ? 1 : (int)min((int64_t)kGroup, a.nr_subgrids - first); // the last group may be short
+        int parts = nseg;
+        if (nseg == 0 && lane < members) {
+            const int s = subgrid(lane), nc = a.ext ? a.ext[s].channel_end - a.ext[s].channel_begin : a.C;
+            const int64_t ntiles = (int64_t)a.md[s].nr_timesteps * nc / kTile;
+            parts = (int)max((int64_t)1, min((int64_t)members, ntiles / kSegTiles));
+        }
+        const int seg = nseg > 0 ? item - first * nseg : q - lane + (q < lane ? members : 0);
+        unsigned todo = __ballot_sync(0xffffffffu, seg < parts && lane < members); // q among them
+        for (int j = q; todo != 0; todo &= ~(1u << j)) {
+            if ((todo >> j & 1u) == 0) { // after the claim's own
+                j = __ffs((int)todo) - 1;
+                si = load_subgrid(a, subgrid(j));
+            }
+            const int sj = subgrid(j), segj = __shfl_sync(0xffffffffu, seg, j), partsj = __shfl_sync(0xffffffffu, parts, j);
             if (!si.ok) {
                 if (lane == 0) flag_status(a.status, kStatusBadPlan);
                 continue;
             }
             const int nc = si.c1 - si.c0;
             if (nc == 0 || si.T == 0) continue;
-            const char *px = reinterpret_cast<const char *>(a.subgrids + (size_t)s * 4 * a.S * a.S);
+            const char *px = reinterpret_cast<const char *>(a.subgrids + (size_t)sj * 4 * a.S * a.S);
             const char *j1 = reinterpret_cast<const char *>(a.aterms + ((size_t)si.aterm * a.nr_stations + si.st1) * jones);
             const char *j2 = reinterpret_cast<const char *>(a.aterms + ((size_t)si.aterm * a.nr_stations + si.st2) * jones);
             for (size_t o = (size_t)lane * 128; o < jones * 16; o += 32 * 128) {
@@ -327,7 +371,7 @@ __device__ __forceinline__ void scout_role(const KernelArgs &a, int nseg, Head *
                 if (lane == 0) atomicAdd(a.fallback, 1);
                 continue;
             }
-            it.s = s;
+            it.s = sj;
             it.row0 = si.row0;
             it.c0 = si.c0;
             it.nc = nc;
@@ -336,18 +380,10 @@ __device__ __forceinline__ void scout_role(const KernelArgs &a, int nseg, Head *
             it.st2 = si.st2;
             it.aterm = si.aterm;
             const int ntiles = (it.nvis + kTile - 1) / kTile;
-            it.t_begin = (int)((int64_t)ntiles * seg / nseg);
-            it.t_end = (int)((int64_t)ntiles * (seg + 1) / nseg);
-            if (it.t_begin >= it.t_end) continue;
+            it.t_begin = (int)((int64_t)ntiles * segj / partsj);
+            it.t_end = (int)((int64_t)ntiles * (segj + 1) / partsj);
+            if (it.t_begin < it.t_end) publish(it);
         }
-        if (k > 0) tc_wait(&head->item_free, (k - 1) & 1, abort, a.status);
-        __syncwarp();
-        if (lane == 0) {
-            head->item = it;
-            mbar_arrive(&head->item_full);
-        }
-        ++k;
-        if (it.stop) return;
     }
 }
 
@@ -636,9 +672,9 @@ cudaError_t launch(const KernelArgs &args, cudaStream_t stream) {
     int64_t blocks = launch_device().sms;
     if (a.share_den > 1) blocks = blocks / a.share_den > 0 ? blocks / a.share_den : 1;
     if (a.max_ctas > 0 && blocks > a.max_ctas) blocks = a.max_ctas;
-    // few subgrids: their tiles are shared out over the CTAs
-    const int nseg = a.nr_subgrids >= blocks ? 1 : (int)(blocks / a.nr_subgrids < 16 ? blocks / a.nr_subgrids : 16);
-    if (blocks > a.nr_subgrids * nseg) blocks = a.nr_subgrids * nseg;
+    // few subgrids: their tiles are shared out over the CTAs; see scout_role
+    const int nseg = a.nr_subgrids >= blocks ? 0 : (int)(blocks / a.nr_subgrids < 16 ? blocks / a.nr_subgrids : 16);
+    if (nseg > 0 && blocks > a.nr_subgrids * nseg) blocks = a.nr_subgrids * nseg;
     kern<<<(unsigned)blocks, kThreads, smem, stream>>>(a, nseg);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     return launch_degridder_unfit(a, stream); // what the expansion does not hold for

@@ -83,6 +83,31 @@ def test_degridder_tiles_shared_out(oracle_mod, idg, subgrids):
     _degrid(_case(24, [40] * subgrids, 10, seed=subgrids), oracle_mod, f"{subgrids} subgrids", TOL)
 
 
+@pytest.mark.parametrize("S", [24, 48])
+@pytest.mark.parametrize("subgrids", [153, 158])
+def test_degridder_long_subgrids_shared_out(idg, S, subgrids):
+    """Long subgrids are cut into segments that their neighbours' claims take.  A
+    visibility's arithmetic does not depend on the cut, so the same subgrids in
+    calls of a few (cut another way) give the same bits; one long subgrid is
+    wider than the expansion holds for, and the last group is not full."""
+    tiles = [1, 31, 32, 33, 48, 1, 1, 63, 64, 65, 80, 1, 200]
+    lengths = [max(1, 8 * tiles[i % len(tiles)] + (i % 3) - 1) if i % 2 or i > 140 else 5 for i in range(subgrids)]
+    c = _case(S, lengths, 16, seed=subgrids)
+    long = int(np.argmax(np.asarray(lengths) > 400))
+    rows = slice(int(c["md"]["time_offset"][long]), int(c["md"]["time_offset"][long]) + lengths[long])
+    c["uvw"][rows, 2] += (8000.0 * np.sin(np.arange(lengths[long]))).astype(np.float32)
+    sp = spec_for(c["G"], S, c["C"], c["ns"], 1, c["img"])
+
+    def run(lo, hi):
+        return degrid_gpu(sp, c["md"][lo:hi], c["uvw"], c["k"], c["sub"][lo:hi], c["taper"], c["at"],
+                          c["uvw"].shape[0], L.VARIANT_BATCHED)
+
+    whole = run(0, subgrids)
+    assert np.all(np.abs(whole).sum(axis=2) > 0)
+    parts = sum(run(lo, min(lo + 40, subgrids)) for lo in range(0, subgrids, 40))
+    assert np.array_equal(whole, parts)
+
+
 def _wide(image_size):
     """Subgrids the expansion does not hold for, between others that it holds for."""
     c = _case(32, [40, 40, 40, 40], 8, seed=3, image_size=image_size)
