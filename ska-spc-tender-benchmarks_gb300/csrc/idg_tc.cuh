@@ -143,16 +143,18 @@ __device__ __forceinline__ void tc_offset(int X, int S, int G, float &hi, float 
 
 // Whether the expansion holds for a (valid) subgrid; NT threads (whole warps,
 // of consecutive numbers) call it and get the same answer, `sync` being their barrier.
-// `scratch`: five words of shared memory.  Only the ranges of u, v, w and of
+// `scratch`: five words of shared memory, not used by a single warp.  Only the ranges of u, v, w and of
 // the wavenumbers enter.
 template <int NT, typename Sync>
 __device__ inline bool tc_fits(const KernelArgs &a, const SubgridInfo &si, unsigned *scratch, TcSubgrid *out,
                                Sync sync) {
     const TcConst &tc = a.tc;
     const int tid = threadIdx.x % NT, nt = NT;
-    sync();
-    if (tid < 5) scratch[tid] = 0u;
-    sync();
+    if constexpr (NT > 32) {
+        sync();
+        if (tid < 5) scratch[tid] = 0u;
+        sync();
+    }
     unsigned m[5] = {0u, 0u, 0u, 0u, 0u}; // max of ord(w), ord(-w), ord(k), ord(-k), |u| |v| |w| as bits
     for (int t = tid; t < si.T; t += nt) {
         const float *p = a.uvw + 3 * ((int64_t)si.row0 + t);
@@ -168,13 +170,17 @@ __device__ inline bool tc_fits(const KernelArgs &a, const SubgridInfo &si, unsig
     }
 #pragma unroll
     for (int i = 0; i < 5; ++i) {
-        const unsigned r = __reduce_max_sync(0xffffffffu, m[i]);
-        if ((tid & 31) == 0 && r) atomicMax(&scratch[i], r);
+        m[i] = __reduce_max_sync(0xffffffffu, m[i]);
+        if (NT > 32 && (tid & 31) == 0 && m[i]) atomicMax(&scratch[i], m[i]);
     }
-    sync();
-    const float wmax = tc_unord(scratch[0]), wmin = -tc_unord(scratch[1]);
-    const float kmax = tc_unord(scratch[2]), kmin = -tc_unord(scratch[3]);
-    const float reach = __uint_as_float(scratch[4]);
+    if constexpr (NT > 32) {
+        sync();
+#pragma unroll
+        for (int i = 0; i < 5; ++i) m[i] = scratch[i];
+    }
+    const float wmax = tc_unord(m[0]), wmin = -tc_unord(m[1]);
+    const float kmax = tc_unord(m[2]), kmin = -tc_unord(m[3]);
+    const float reach = __uint_as_float(m[4]);
     const float g[4] = {kmin * wmin, kmin * wmax, kmax * wmin, kmax * wmax};
     const float gmin = fminf(fminf(g[0], g[1]), fminf(g[2], g[3])) * (1.f / kTwoPiF);
     const float gmax = fmaxf(fmaxf(g[0], g[1]), fmaxf(g[2], g[3])) * (1.f / kTwoPiF);

@@ -108,6 +108,32 @@ def test_degridder_long_subgrids_shared_out(idg, S, subgrids):
     assert np.array_equal(whole, parts)
 
 
+@pytest.mark.parametrize("S,subgrids", [(24, 160), (24, 161), (24, 191), (48, 45), (48, 64)])
+@pytest.mark.parametrize("even", [False, True])
+def test_gridder_longest_first(idg, S, subgrids, even):
+    """More items than CTAs are taken by length.  A subgrid's sum does not depend on
+    when it is taken, so calls of a few subgrids (in the plan's order) give the
+    same bits; groups of 32 that are full, of one and of less, lengths with ties
+    and zeros, and one subgrid that the expansion does not hold for."""
+    rng = np.random.default_rng(subgrids)
+    lengths = [20] * subgrids if even else [int(x) for x in rng.choice([0, 1, 7, 40, 40, 90, 300], subgrids)]
+    if not even:
+        lengths[3] = 40
+    c = _case(S, lengths, 9, seed=subgrids)
+    rows = slice(int(c["md"]["time_offset"][3]), int(c["md"]["time_offset"][3]) + lengths[3])
+    c["uvw"][rows, 2] += (8000.0 * np.sin(np.arange(lengths[3]))).astype(np.float32)
+    sp = spec_for(c["G"], S, c["C"], c["ns"], 1, c["img"])
+    few = 30 if S > 32 else 120
+
+    def run(lo, hi):
+        return grid_gpu(sp, c["md"][lo:hi], c["uvw"], c["k"], c["vis"], c["taper"], c["at"], L.VARIANT_BATCHED)
+
+    whole = run(0, subgrids)
+    parts = np.concatenate([run(lo, min(lo + few, subgrids)) for lo in range(0, subgrids, few)])
+    assert np.array_equal(whole, parts)
+    assert all((np.abs(whole[i]).max() > 0) == (lengths[i] > 0) for i in range(subgrids))
+
+
 def _wide(image_size):
     """Subgrids the expansion does not hold for, between others that it holds for."""
     c = _case(32, [40, 40, 40, 40], 8, seed=3, image_size=image_size)
