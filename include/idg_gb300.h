@@ -470,7 +470,8 @@ typedef struct idg_cycle_timing {
  * gridding (the first copy in is small, so the kernels start early, and each
  * later copy finishes while the previous chunk is gridded, for copy rates of
  * 1.6x the rate the kernels consume) and shrink by 1.6x while degridding (the
- * last copy out is small), at least 1024 subgrids each; IDG_CHUNKS_ADAPTIVE:
+ * last copy out is small), at least a quarter of the plan or 1024 subgrids each
+ * and never under 512; IDG_CHUNKS_ADAPTIVE:
  * the same with the ratio learned from the previous cycle; 0: one chunk.  uvw
  * rows travel with their chunk.  Device buffers are kept between calls of
  * the same sizes and freed by idg_release_buffers().  Pinned host buffers

@@ -61,11 +61,13 @@ struct Chunk {
 // Subgrid boundaries 0 = b0 < b1 < ... = n.  chunk > 0: equal chunks of that
 // many subgrids; IDG_CHUNKS_AUTO / IDG_CHUNKS_ADAPTIVE: `pieces` chunks
 // whose sizes grow by `ratio` from one to the next (`growing`) or shrink by
-// it (otherwise), chunks under kMinChunk subgrids merged into their
-// neighbour; anything else: one chunk.  A growing chunk's copy keeps ahead of
-// the previous chunk's kernels while the copy rate is at least `ratio` times
-// the rate the kernels consume visibilities (about 61 GB/s for the config-2
-// gridder: at ratio 1.6, copies at 98 GB/s or more suffice).
+// it (otherwise), chunks under a quarter of the plan, but at least 512 and at most
+// kMinChunk subgrids, merged into their neighbour; anything else: one chunk.
+// (Chunks of 512: a cycle of 2,016 subgrids takes 2.08 ms in two chunks, 2.21 in
+// one, 2.22 in four; 8,010 take 5.20 in four of 1,024 or more, 5.27 in five.)  A
+// growing chunk's copy keeps ahead of the previous chunk's kernels while the copy
+// rate is at least `ratio` times the rate the kernels consume visibilities (the
+// gridder takes about 180 GB/s at S = 32).
 constexpr int64_t kMinChunk = 1024;
 constexpr int kAutoChunks = 10;
 constexpr int kRunChunks = 4; // see run_cycles
@@ -75,13 +77,14 @@ std::vector<int64_t> chunk_bounds(int64_t n, int64_t chunk, bool growing, double
     std::vector<int64_t> b{0};
     if (chunk == IDG_CHUNKS_AUTO || chunk == IDG_CHUNKS_ADAPTIVE) {
         const int k = pieces;
+        const int64_t least = std::max<int64_t>(512, std::min<int64_t>(kMinChunk, n / 4));
         double total = 0;
         for (int i = 0; i < k; ++i) total += std::pow(ratio, i);
         double acc = 0;
         for (int i = 0; i < k; ++i) {
             acc += std::pow(ratio, growing ? i : k - 1 - i);
             const int64_t e = i == k - 1 ? n : (int64_t)(n * acc / total + 0.5);
-            if (e - b.back() >= kMinChunk) b.push_back(e);
+            if (e - b.back() >= least) b.push_back(e);
         }
         if (b.size() == 1) b.push_back(n);
         b.back() = n; // the last chunk takes what the merges left
