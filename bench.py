@@ -19,9 +19,12 @@ Printed (rank 0, one JSON line):
           idg_imaging_cycles() call, each cycle's copies in running while the
           cycle before it degrids; `single_cycle` beside it is one
           idg_imaging_cycle() call per step
-  roofline of the gridder and the degridder: 17 FMA (34 flop) per
-          pixel-visibility over the measured FP32 FMA peak of this device; the
-          top-level figures are those of the kernel with the larger time share
+  roofline of the gridder and the degridder: on the tensor cores, the three
+          fp16 products of split operands that stand for the 32 flop of a
+          pixel-visibility's four complex MACs, over the measured dense bf16
+          rate (fp16 runs at the same); for the other kernels 17 FMA (34 flop)
+          over the measured FP32 FMA peak; the top-level figures are those of
+          the kernel with the larger time share
   cpu_baseline the reference's CPU algorithm (the oracle's float restatement of
           its OpenMP launchers) on a bounded sample of the same workload
   serving p50 / p99 job latency and Mvis/s of a Poisson stream of gridding and
@@ -51,12 +54,12 @@ sys.path.insert(0, os.path.join(ROOT, "ska-spc-tender-benchmarks_gb300"))
 
 METRIC = "Mvis/s grid+degrid vs plain GPU form at ≤1e-5 rel err; p50/p99 job latency"
 FLOP_PER_PIXVIS = 34.0  # 16 FMA of the four complex MACs + 1 FMA of the phase
+TENSOR_FLOP_PER_PIXVIS = 96.0  # the 16 FMA as three products: hi hi, hi lo, lo hi
 # DRAM bytes (read + write) per subgrid of one batched kernel launch, S = 32, 16
-# channels x 128 timesteps: ncu capture of one launch on the first 8192
-# subgrids of the config-2 plan with the tuned mirror-quad shapes (gridder
-# shape 24: 690.4 MB read + 245.2 MB written; degridder shape 34: 418.4 MB
-# read + 490.1 MB written), divided by 8192.
-DRAM_BYTES_PER_SUBGRID = {"gridder": 114213.0, "degridder": 110901.0}
+# channels x 128 timesteps: ncu captures of one launch on 4,416 such subgrids with
+# the tensor-core shapes (gridder 309.8 MB read + 118.2 MB written, degridder
+# 161.1 MB + 234.7 MB), divided by 4,416.
+DRAM_BYTES_PER_SUBGRID = {"gridder": 96921.0, "degridder": 89623.0}
 
 
 def parse():
@@ -578,17 +581,29 @@ def run_ours(args, rank, world, local_rank):
     stream.synchronize()
     parts = np.array([[ev[j].elapsed_time(ev[j + 1]) for j in range(5)]])
 
-    # roofline (FP32 FMA bound) of the gridder and the degridder; the JSON's
-    # top-level figures are those of the kernel with the larger time share
+    # roofline of the gridder and the degridder; the JSON's top-level figures are
+    # those of the kernel with the larger time share
     pixvis = float(nvis) * S * S
     grid_ms = float(np.mean(parts[:, 0]))
     degrid_ms = float(np.mean(parts[:, 4]))
-    peak = ops.measure_fp32_peak()
+    fp32_peak = ops.measure_fp32_peak()
+    from idg_gb300 import tuning
+
+    last = [n - 1 for n in tuning.num_shapes()]
+    tensor = [variant != ops.VARIANT_PLAIN and a == b for a, b in zip(tuning.get_shapes(S), last)]
+    tensor_peak, tensor_source = 1.9e15, "fallback: 1.9 PFLOP/s dense bf16"
+    try:
+        with open(os.path.join(ROOT, "MEASURED_PEAKS.json")) as f:
+            tensor_peak, tensor_source = float(json.load(f)["bf16_tflops"]) * 1e12, "MEASURED_PEAKS.json bf16_tflops"
+    except (OSError, ValueError, KeyError):
+        pass
     per_kernel = {}
-    for name, ms in (("gridder", grid_ms), ("degridder", degrid_ms)):
-        ach = FLOP_PER_PIXVIS * pixvis / (ms * 1e-3)
-        traffic = DRAM_BYTES_PER_SUBGRID[name] * N if S == 32 else None
-        per_kernel[name] = {"achieved": ach / 1e12, "frac": ach / peak, "ms": ms, "traffic": traffic}
+    for name, ms, tc in (("gridder", grid_ms, tensor[0]), ("degridder", degrid_ms, tensor[1])):
+        ach = (TENSOR_FLOP_PER_PIXVIS if tc else FLOP_PER_PIXVIS) * pixvis / (ms * 1e-3)
+        top = tensor_peak if tc else fp32_peak
+        traffic = DRAM_BYTES_PER_SUBGRID[name] * N if S == 32 and tc else None
+        per_kernel[name] = {"bound": "tensor" if tc else "fp32", "achieved": ach / 1e12, "peak": top / 1e12,
+                            "frac": ach / top, "ms": ms, "traffic": traffic}
     dom = "degridder" if degrid_ms > grid_ms else "gridder"
     # the measured FFMA peak against 128 FP32 lanes x 2 flop per SM clock, at
     # the SM clock sampled over the timed region (the microbenchmark itself
@@ -598,21 +613,22 @@ def run_ours(args, rank, world, local_rank):
     theory = props.multi_processor_count * 128 * 2 * sm_mhz * 1e6 if sm_mhz else None
     peak_check = {"sms": props.multi_processor_count, "fp32_lanes_per_sm": 128, "sm_mhz": sm_mhz,
                   "lanes_x_2_x_clock_tflops": theory / 1e12 if theory else None,
-                  "measured_over_lanes_x_2_x_clock": peak / theory if theory else None}
+                  "fp32_peak": fp32_peak / 1e12,
+                  "measured_over_lanes_x_2_x_clock": fp32_peak / theory if theory else None}
     roof = {
-        "bound": "fp32",
+        "bound": per_kernel[dom]["bound"],
         "kernel": dom,
         "achieved": per_kernel[dom]["achieved"],
-        "peak": peak / 1e12,
+        "peak": per_kernel[dom]["peak"],
         "unit": "TFLOP/s",
         "frac": per_kernel[dom]["frac"],
         "traffic": per_kernel[dom]["traffic"],
-        "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of one launch on the first 8192 "
-                          "subgrids of this plan, scaled by subgrids (the kernels stream each subgrid's data once)",
-        "peak_source": "measured in this run: FFMA microbenchmark idg_measure_fp32_peak (MEASURED_PEAKS.json "
-                       "carries HBM and bf16 figures, no FP32 FMA figure); the SFU bound (16 sin/cos per SM clock, 2 per "
-                       "pixel-visibility) is within 2% of the FMA bound on GB300",
-        "algorithmic": "34 flop (17 FMA) + 1 sincos per pixel-visibility; %.3g pixel-visibilities per launch" % pixvis,
+        "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of one launch on 4,416 "
+                          "subgrids of this shape, scaled by subgrids (the kernels stream each subgrid's data once)",
+        "peak_source": "tensor: " + tensor_source + " (fp16 runs at the bf16 rate); fp32: measured in this run, FFMA "
+                       "microbenchmark idg_measure_fp32_peak",
+        "algorithmic": "tensor: three fp16 products for the 32 flop of four complex MACs, 96 flop per pixel-visibility; "
+                       "fp32: 34 flop (17 FMA) + 1 sincos; %.3g pixel-visibilities per launch" % pixvis,
         "peak_check": peak_check,
         "gridder": per_kernel["gridder"],
         "degridder": per_kernel["degridder"],
@@ -623,7 +639,7 @@ def run_ours(args, rank, world, local_rank):
         plan.close()
 
     # imaging step around the cycle: the uv-grid -> image FFT (idg_grid_fft) on
-    # this grid, outside the timed cycle; 4 HBM passes (2 row FFTs, 2 transposes)
+    # this grid, outside the timed cycle; 2 HBM passes (rows, columns)
     imaging = None
     if G <= 8192 and (G & (G - 1)) == 0:
         ge = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
@@ -635,7 +651,7 @@ def run_ours(args, rank, world, local_rank):
             ge[1].record(stream)
         stream.synchronize()
         fft_ms = ge[0].elapsed_time(ge[1]) / 3
-        nbytes = 4 * 2 * grid.numel() * 8
+        nbytes = 2 * 2 * grid.numel() * 8
         hbm_peak = None
         try:
             with open(os.path.join(ROOT, "MEASURED_PEAKS.json")) as f:
@@ -646,7 +662,7 @@ def run_ours(args, rank, world, local_rank):
         imaging = {"grid_fft_ms": fft_ms, "grid": f"1x4x{G}^2",
                    "hbm_bytes": nbytes, "achieved_gbs": ach,
                    "frac_of_measured_hbm": ach / hbm_peak if hbm_peak else None,
-                   "note": "not part of the timed cycle; HBM bytes = 4 passes x (read + write) of the grid"}
+                   "note": "not part of the timed cycle; HBM bytes = 2 passes x (read + write) of the grid"}
 
     # plain form (one step, same data) for the batched / plain ratio
     plain = None
@@ -709,7 +725,9 @@ def run_ours(args, rank, world, local_rank):
         "config": config_block(spec, args.workload, {"variant": args.variant, "parallelism": f"replicas x{world}",
                                                      "tuned_shapes": tune}),
         "e2e": e2e,
-        "gpu_launches": 6 * args.steps,
+        # gridder, FFT, two adder passes, split + FFT, degridder; behind a tensor-core
+        # kernel a general one takes what it leaves
+        "gpu_launches": (6 + sum(tensor)) * args.steps,
         "roofline": roof,
         "cpu_baseline": cpu,
         "plain": plain,

@@ -106,7 +106,7 @@ typedef struct idg_benchmark_result {
 
 /* Kernel variants */
 #define IDG_VARIANT_PLAIN 0   /* one CTA per subgrid, one sincos per pixel-visibility */
-#define IDG_VARIANT_BATCHED 1 /* persistent CTAs over a cost-sorted work list, TMA-staged inputs */
+#define IDG_VARIANT_BATCHED 1 /* persistent CTAs over a work list; tensor cores where the size allows */
 
 /* ------------------------------------------------------------------ */
 /* Library                                                            */
@@ -134,8 +134,8 @@ IDG_API int idg_gridder(const idg_params *params, int variant, int64_t nr_subgri
 
 /* The batched gridder (IDG_VARIANT_BATCHED of idg_gridder), for callers that
  * may not allocate device memory.  No counterpart in the reference.
- * idg_gridder() obtains its two scratch words (work counter, check word) with
- * cudaMalloc on first use; this entry point keeps them in a 256-byte static
+ * idg_gridder() obtains its scratch words (work counter, check word, hand-over
+ * between its kernels) with cudaMalloc on first use; this entry point keeps them in a 256-byte static
  * device array of the library instead and calls no allocator.  Same arguments
  * and result as idg_gridder().  Limits: at most 2^30 subgrids; calls on one
  * device share the array, so calls whose kernels could overlap on the GPU
@@ -580,7 +580,8 @@ IDG_API int idg_reference_dataset(int64_t grid_size, int64_t subgrid_size, int64
 /* The batched gridder and degridder are compiled in several launch shapes
  * (threads per CTA, pixels, quads or octets per thread, staging tile, CTAs
  * per SM).  Until set here or by idg_autotune(), a subgrid size uses the
- * shapes measured fastest for it on GB300 (the mirror-quad kernels where
+ * shapes measured fastest for it on GB300 (the tensor-core kernels, the last
+ * shape of each, for even sizes from 8 to 64; else the mirror-quad kernels where
  * their layout fits the size).  No counterpart in the reference. */
 IDG_API int idg_batched_shapes(int *gridder_shapes, int *degridder_shapes);
 IDG_API int idg_set_batched_shapes(int subgrid_size, int gridder_shape, int degridder_shape);
