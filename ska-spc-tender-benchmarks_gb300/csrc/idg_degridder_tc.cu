@@ -30,7 +30,8 @@
 // share the SM's four schedulers.  28 subgrids of 64 x 16 in one call: 25 us
 // against 115 us.
 // Subgrids larger than 32 are done in blocks of at most 32 x 32 pixels, the
-// later blocks adding to the visibilities written by the first.
+// later blocks adding to the visibilities written by the first, once all results
+// of the block before are stored.
 #include "idg_tc.cuh"
 #include "idg_internal.h"
 
@@ -533,6 +534,11 @@ __device__ __forceinline__ void result_role(const KernelArgs &a, Head *head, con
                         o[2 * p + 1] = (e + f) * job.inv;
                     }
                     if (job.add) {
+                        // With an odd number of tiles the block before had this one in the
+                        // other warpgroup: its stores come first.  (Its threads are past that
+                        // job or ahead of this one in the products' order, so they never wait
+                        // for this one.)
+                        tc_wait(&head->job_free[buf ^ 1], ((j - 1) >> 1) & 1, abort, a.status);
                         const float4 e = dst[0], f = dst[1];
                         o[0] += e.x, o[1] += e.y, o[2] += e.z, o[3] += e.w;
                         o[4] += f.x, o[5] += f.y, o[6] += f.z, o[7] += f.w;
