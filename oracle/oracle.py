@@ -99,7 +99,7 @@ def build(with_ref: bool | None = None) -> None:
         if build_type != "-O2":
             _compile_variant(build_type)
     if with_ref is None:
-        with_ref = bool(REFERENCE_DIR) and os.path.isdir(REFERENCE_DIR)
+        with_ref = bool(REFERENCE_DIR) and os.path.isdir(os.path.join(REFERENCE_DIR, "gridding", "src"))
     if with_ref:
         g = os.path.join(REFERENCE_DIR, "gridding")
         ref_src = [os.path.join(g, "src", f) for f in ("gridding_benchmark.cpp", "degridding_benchmark.cpp",

@@ -1,0 +1,8 @@
+"""The oracle's build without the reference's sources."""
+
+
+def test_an_empty_reference_folder_counts_as_none(oracle_mod, monkeypatch, tmp_path):
+    monkeypatch.setattr(oracle_mod, "REFERENCE_DIR", str(tmp_path))
+    monkeypatch.setattr(oracle_mod, "REF_SO", str(tmp_path / "ref.so"))
+    oracle_mod.build()
+    assert list(tmp_path.iterdir()) == []
