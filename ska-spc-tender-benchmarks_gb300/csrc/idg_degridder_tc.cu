@@ -137,9 +137,12 @@ __device__ __forceinline__ uint32_t op_row(int y, int p) { return (uint32_t)(16 
 
 // S' of the block's pixels (x0 + x, y0 + y) into the operand layout: first the
 // largest magnitude, then scaled and split.  Returns the reciprocal scale.
+// given_up: a wait ran out, perhaps one for this operand or its job; the same
+// answer for all threads.
 template <int ROWS>
 __device__ __forceinline__ float stage_block(const KernelArgs &a, const Item &si, Head *head, const Shape &sh, int x0,
-                                             int y0, unsigned char *bh, const float4 *axis, const float2 *ntab) {
+                                             int y0, unsigned char *bh, const float4 *axis, const float2 *ntab,
+                                             bool *given_up) {
     const TcSubgrid &sg = si.sg;
     const int s = si.s;
     const int tid = threadIdx.x, S = a.S, S2 = S * S, Sh = S / 2;
@@ -151,8 +154,13 @@ __device__ __forceinline__ float stage_block(const KernelArgs &a, const Item &si
     const int kp = sh.kx / 2, items = kp * sh.nq * ROWS;
     unsigned char *bl = bh + Op<ROWS>::bytes * sh.nq, *b1 = bl + Op<ROWS>::bytes * sh.nq;
     gen_sync(); // the previous block's readers of max_bits are past it
-    if (tid == 0) head->max_bits = 0u;
+    if (tid == 0) {
+        head->max_bits = 0u;
+        head->gen_stop = *(volatile int *)&head->abort;
+    }
     gen_sync();
+    *given_up = head->gen_stop != 0;
+    if (*given_up) return 0.f;
     constexpr int kIter = 2; // at most 512 pixel pairs
     cf v[kIter][2][4];
     unsigned m = 0u;
@@ -318,7 +326,8 @@ __device__ __forceinline__ void scout_role(const KernelArgs &a, int nseg, Head *
     uint32_t k = 0;
     auto publish = [&](const Item &it) {
         if (k > 0) tc_wait(&head->item_free, (k - 1) & 1, abort, a.status);
-        __syncwarp();
+        // a wait that was given up leaves the item to those who may be reading it
+        if (__any_sync(0xffffffffu, *abort)) return;
         if (lane == 0) {
             head->item = it;
             mbar_arrive(&head->item_full);
@@ -415,7 +424,10 @@ __device__ __forceinline__ void factor_role(const KernelArgs &a, Head *head, con
                 tc_wait(&head->b_free[buf], ((j >> 1) - 1) & 1, abort, a.status);
                 tc_wait(&head->job_free[buf], ((j >> 1) - 1) & 1, abort, a.status);
             }
-            const float inv = stage_block<ROWS>(a, it, head, sh, x0, y0, smem + L.b + buf * L.bset, axis, ntab);
+            bool given_up;
+            const float inv =
+                stage_block<ROWS>(a, it, head, sh, x0, y0, smem + L.b + buf * L.bset, axis, ntab, &given_up);
+            if (given_up) return; // the others may be reading the job that would be overwritten
             if (tid == 0)
                 head->job[buf] = Job{0, it.nc, it.t_begin, it.t_end, it.c0, it.row0, y0, block > 0, it.nvis, it.sg,
                                      inv * kTcTruncation};
@@ -608,7 +620,7 @@ __device__ __forceinline__ void issue_role(const KernelArgs &a, Head *head, cons
         if (lead) umma_commit(&head->b_free[buf]);
         __syncwarp();
     }
-    if (lead && *abort) { // let products in flight end (bounded) before their memory goes
+    if (lead && n > 0) { // products in flight end (bounded) before their memory goes, also where a reader gave up
         umma_commit(&head->drain);
         mbar_wait_bounded(&head->drain, 0, kTcWaitNs);
     }

@@ -232,7 +232,8 @@ __device__ __forceinline__ void scout_role(const KernelArgs &a, Head *head, cons
             it.aterm = si.aterm;
         }
         if (k > 0) tc_wait(&head->item_free, (k - 1) & 1, abort, a.status);
-        __syncwarp();
+        // a wait that was given up leaves the item to those who may be reading it
+        if (__any_sync(0xffffffffu, *abort)) return;
         if (lane == 0) {
             head->item = it;
             mbar_arrive(&head->item_full);
@@ -648,7 +649,7 @@ __device__ __forceinline__ void issue_role(const KernelArgs &a, Head *head, cons
         if (lead) umma_commit(&head->d_full[buf]);
         __syncwarp();
     }
-    if (lead && *abort) { // let products in flight end (bounded) before their memory goes
+    if (lead && gs > 0) { // products in flight end (bounded) before their memory goes, also where a reader gave up
         umma_commit(&head->drain);
         mbar_wait_bounded(&head->drain, 0, kTcWaitNs);
     }
