@@ -69,7 +69,8 @@ struct Head {
     uint64_t item_full, item_free;
     uint64_t drain;
     uint32_t tmem;
-    int abort, gen_stop;
+    TcWatch watch;
+    int gen_stop;
     unsigned max_bits;
     unsigned scratch[5];
     Item item;
@@ -156,7 +157,7 @@ __device__ __forceinline__ float stage_block(const KernelArgs &a, const Item &si
     gen_sync(); // the previous block's readers of max_bits are past it
     if (tid == 0) {
         head->max_bits = 0u;
-        head->gen_stop = *(volatile int *)&head->abort;
+        head->gen_stop = ((volatile TcWatch *)&head->watch)->abort;
     }
     gen_sync();
     *given_up = head->gen_stop != 0;
@@ -320,14 +321,14 @@ __device__ __forceinline__ void issue_rows(uint32_t d, uint32_t am, uint32_t bh,
 //    5 of 880 us, of one tile each 6 of 228.  Claims for every segment, the empty
 //    ones too, made that last call 299 us.
 __device__ __forceinline__ void scout_role(const KernelArgs &a, int nseg, Head *head) {
-    volatile int *abort = &head->abort;
+    volatile TcWatch *watch = &head->watch;
     const int lane = threadIdx.x & 31;
     const size_t jones = (size_t)a.S * a.S * 2; // float4 per matrix plane
     uint32_t k = 0;
     auto publish = [&](const Item &it) {
-        if (k > 0) tc_wait(&head->item_free, (k - 1) & 1, abort, a.status);
+        if (k > 0) tc_wait(&head->item_free, (k - 1) & 1, watch, a.status);
         // a wait that was given up leaves the item to those who may be reading it
-        if (__any_sync(0xffffffffu, *abort)) return;
+        if (__any_sync(0xffffffffu, watch->abort)) return;
         if (lane == 0) {
             head->item = it;
             mbar_arrive(&head->item_full);
@@ -336,7 +337,7 @@ __device__ __forceinline__ void scout_role(const KernelArgs &a, int nseg, Head *
     };
     for (;;) {
         int item = 0;
-        if (lane == 0) item = *abort ? INT32_MAX : atomicAdd(a.work_counter, 1);
+        if (lane == 0) item = watch->abort ? INT32_MAX : atomicAdd(a.work_counter, 1);
         item = __shfl_sync(0xffffffffu, item, 0);
         Item it{};
         if (item >= a.nr_subgrids * (nseg > 0 ? nseg : 1)) {
@@ -362,6 +363,7 @@ __device__ __forceinline__ void scout_role(const KernelArgs &a, int nseg, Head *
                 j = __ffs((int)todo) - 1;
                 si = load_subgrid(a, subgrid(j));
             }
+            if (lane == 0) watch->looked = global_timer_ns();
             const int sj = subgrid(j), segj = __shfl_sync(0xffffffffu, seg, j), partsj = __shfl_sync(0xffffffffu, parts, j);
             if (!si.ok) {
                 if (lane == 0) flag_status(a.status, kStatusBadPlan);
@@ -404,12 +406,12 @@ __device__ __forceinline__ void factor_role(const KernelArgs &a, Head *head, con
     const float4 *axis = reinterpret_cast<const float4 *>(smem + L.axis);
     const float2 *ntab = reinterpret_cast<const float2 *>(smem + L.ntab);
     const float4 *chan = reinterpret_cast<const float4 *>(smem + L.chan);
-    volatile int *abort = &head->abort;
+    volatile TcWatch *watch = &head->watch;
     const int tid = threadIdx.x, wg = tid >> 7, lane = tid & 127;
     uint32_t n = 0, uses = 0, j = 0; // tiles so far, this warpgroup's, jobs so far
     for (uint32_t k = 0;; ++k) {
-        tc_wait(&head->item_full, k & 1, abort, a.status);
-        if (tid == 0) head->gen_stop = head->item.stop || *abort; // one answer for all
+        tc_wait(&head->item_full, k & 1, watch, a.status);
+        if (tid == 0) head->gen_stop = head->item.stop || watch->abort; // one answer for all
         gen_sync();
         const Item it = head->item;
         const bool stop = head->gen_stop != 0;
@@ -421,8 +423,8 @@ __device__ __forceinline__ void factor_role(const KernelArgs &a, Head *head, con
             const int x0 = (block % sh.nb) * sh.bs, y0 = (block / sh.nb) * sh.bs;
             const uint32_t buf = j & 1;
             if (j >= 2) {
-                tc_wait(&head->b_free[buf], ((j >> 1) - 1) & 1, abort, a.status);
-                tc_wait(&head->job_free[buf], ((j >> 1) - 1) & 1, abort, a.status);
+                tc_wait(&head->b_free[buf], ((j >> 1) - 1) & 1, watch, a.status);
+                tc_wait(&head->job_free[buf], ((j >> 1) - 1) & 1, watch, a.status);
             }
             bool given_up;
             const float inv =
@@ -446,7 +448,7 @@ __device__ __forceinline__ void factor_role(const KernelArgs &a, Head *head, con
                 float hi, lo;
                 tc_slope(v.k.x, v.k.y, v.u, it.sg.xh, it.sg.xl, hi, lo);
                 const float d = kTwoPiF * tc_delta(v.k.z, v.k.w, v.w, it.sg.mid);
-                if (uses > 0) tc_wait(&head->a_free[wg], (uses - 1) & 1, abort, a.status);
+                if (uses > 0) tc_wait(&head->a_free[wg], (uses - 1) & 1, watch, a.status);
                 __syncwarp();
                 tmem_fence_after();
                 store_factors(tl + kColA + kColsA * wg, sh, axis + x0, hi, lo * kTwoPiF, d, it.sg.cross != 0);
@@ -458,7 +460,7 @@ __device__ __forceinline__ void factor_role(const KernelArgs &a, Head *head, con
     }
     // the end, for the other roles
     const uint32_t buf = j & 1;
-    if (j >= 2) tc_wait(&head->job_free[buf], ((j >> 1) - 1) & 1, abort, a.status);
+    if (j >= 2) tc_wait(&head->job_free[buf], ((j >> 1) - 1) & 1, watch, a.status);
     gen_sync();
     if (tid == 0) {
         head->job[buf].stop = 1;
@@ -472,14 +474,14 @@ __device__ __forceinline__ void result_role(const KernelArgs &a, Head *head, con
                                             unsigned char *smem, uint32_t tl) {
     const float4 *axis = reinterpret_cast<const float4 *>(smem + L.axis);
     const float4 *chan = reinterpret_cast<const float4 *>(smem + L.chan);
-    volatile int *abort = &head->abort;
+    volatile TcWatch *watch = &head->watch;
     const int wg = (threadIdx.x >> 7) & 1, lane = threadIdx.x & 127;
     uint32_t n = 0, uses = 0;
     for (uint32_t j = 0;; ++j) {
         const uint32_t buf = j & 1;
-        tc_wait(&head->job_full[buf], (j >> 1) & 1, abort, a.status);
+        tc_wait(&head->job_full[buf], (j >> 1) & 1, watch, a.status);
         __syncwarp();
-        if (__any_sync(0xffffffffu, *abort)) return;
+        if (__any_sync(0xffffffffu, watch->abort)) return;
         const Job job = head->job[buf];
         if (job.stop) return;
         const int nvis = job.nvis;
@@ -504,7 +506,7 @@ __device__ __forceinline__ void result_role(const KernelArgs &a, Head *head, con
                 for (int h = 0; h < sh.nq; ++h) {
                     const float4 *ax = axis + job.y0 + h * ROWS;
                     const uint32_t col = tl + ((r0 + h) % kAcc) * 128u;
-                    tc_wait(&head->d_full[wg][h], uses & 1, abort, a.status);
+                    tc_wait(&head->d_full[wg][h], uses & 1, watch, a.status);
                     __syncwarp();
                     tmem_fence_after();
 #pragma unroll
@@ -550,7 +552,7 @@ __device__ __forceinline__ void result_role(const KernelArgs &a, Head *head, con
                         // other warpgroup: its stores come first.  (Its threads are past that
                         // job or ahead of this one in the products' order, so they never wait
                         // for this one.)
-                        tc_wait(&head->job_free[buf ^ 1], ((j - 1) >> 1) & 1, abort, a.status);
+                        tc_wait(&head->job_free[buf ^ 1], ((j - 1) >> 1) & 1, watch, a.status);
                         const float4 e = dst[0], f = dst[1];
                         o[0] += e.x, o[1] += e.y, o[2] += e.z, o[3] += e.w;
                         o[4] += f.x, o[5] += f.y, o[6] += f.z, o[7] += f.w;
@@ -569,16 +571,16 @@ __device__ __forceinline__ void result_role(const KernelArgs &a, Head *head, con
 template <int ROWS, int KJ, bool CROSS>
 __device__ __forceinline__ void issue_job(const KernelArgs &a, Head *head, const Shape &sh, uint32_t t0, uint32_t b0,
                                           uint32_t n, int tiles, uint32_t lead) {
-    volatile int *abort = &head->abort;
+    volatile TcWatch *watch = &head->watch;
     const uint32_t group = Op<ROWS>::bytes >> 4, set = group * (uint32_t)sh.nq;
     const uint32_t back = kAcc / (uint32_t)sh.nq; // tiles to an accumulator's last user
 #pragma unroll 1
     for (int i = 0; i < tiles; ++i, ++n) {
         const uint32_t w = n & 1, am = t0 + kColA + kColsA * w;
-        tc_wait(&head->a_full[w], (n >> 1) & 1, abort, a.status);
+        tc_wait(&head->a_full[w], (n >> 1) & 1, watch, a.status);
 #pragma unroll 1
         for (uint32_t h = 0; h < (uint32_t)sh.nq; ++h) {
-            if (n >= back) tc_wait(&head->d_free[(n - back) & 1][h], ((n - back) >> 1) & 1, abort, a.status);
+            if (n >= back) tc_wait(&head->d_free[(n - back) & 1][h], ((n - back) >> 1) & 1, watch, a.status);
             tmem_fence_after();
             if (lead) {
                 const uint32_t bh = b0 + h * group;
@@ -595,14 +597,14 @@ __device__ __forceinline__ void issue_job(const KernelArgs &a, Head *head, const
 template <int ROWS>
 __device__ __forceinline__ void issue_role(const KernelArgs &a, Head *head, const Shape &sh, const Layout &L,
                                            unsigned char *smem, uint32_t tm) {
-    volatile int *abort = &head->abort;
+    volatile TcWatch *watch = &head->watch;
     const uint32_t lead = elect_lane(), t0 = warp_uniform(tm);
     uint32_t n = 0;
     for (uint32_t j = 0;; ++j) {
         const uint32_t buf = j & 1;
-        tc_wait(&head->job_full[buf], (j >> 1) & 1, abort, a.status);
+        tc_wait(&head->job_full[buf], (j >> 1) & 1, watch, a.status);
         __syncwarp();
-        if (__any_sync(0xffffffffu, *abort) || warp_uniform(head->job[buf].stop)) break;
+        if (__any_sync(0xffffffffu, watch->abort) || warp_uniform(head->job[buf].stop)) break;
         const uint32_t b0 = warp_uniform(umma_desc_lo(smem_addr(smem + L.b + buf * L.bset), Op<ROWS>::ks));
         const int tiles = (int)warp_uniform(head->job[buf].t_end - head->job[buf].t_begin);
         const bool cross = warp_uniform(head->job[buf].sg.cross) != 0;
@@ -655,7 +657,7 @@ __global__ void __launch_bounds__(kThreads, 1) degridder_tc_kernel(KernelArgs a,
         mbar_init(&head->item_free, kGen);
         mbar_init(&head->drain, 1);
         mbar_init_fence();
-        head->abort = 0;
+        head->watch = TcWatch{0, 0};
     }
     tc_axis_table(a, reinterpret_cast<float4 *>(smem + L.axis), sh.nb * sh.bs / 2 + 16, tid, kThreads);
     tc_n_table(a, reinterpret_cast<float2 *>(smem + L.ntab), tid, kThreads);

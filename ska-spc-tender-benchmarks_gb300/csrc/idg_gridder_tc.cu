@@ -75,7 +75,8 @@ struct Head {
     uint64_t d_full[2], d_free[2]; // accumulators
     uint64_t item_full, item_free, drain;
     uint32_t tmem;
-    int abort, load_stop;
+    TcWatch watch;
+    int load_stop;
     unsigned scratch[5];
     unsigned wmax[2][2];
     Item item;
@@ -181,17 +182,18 @@ __device__ __forceinline__ int subgrid_of(const Claim &c, bool ranked, float *le
 // Takes (subgrid, block) items from the work counter; leaves out what the
 // expansion does not hold for.
 __device__ __forceinline__ void scout_role(const KernelArgs &a, Head *head, const Shape &sh) {
-    volatile int *abort = &head->abort;
+    volatile TcWatch *watch = &head->watch;
     const int lane = threadIdx.x & 31, nblocks = sh.nb * sh.nb, S2 = a.S * a.S;
     const size_t jones = (size_t)S2 * 2;
     const bool ranked = a.nr_subgrids * nblocks > (int64_t)gridDim.x;
-    auto claim = [&] { return lane > 0 ? 0 : *abort ? INT32_MAX : atomicAdd(a.work_counter, 1); };
+    auto claim = [&] { return lane > 0 ? 0 : watch->abort ? INT32_MAX : atomicAdd(a.work_counter, 1); };
     auto look = [&](int c) { return look_up(a, __shfl_sync(0xffffffffu, c, 0), nblocks, ranked); };
     Claim next{};
     int ahead = 0;      // the claim after the next one
     bool eager = false; // down to the short ones
     for (uint32_t k = 0;;) {
         const Claim now = eager ? next : look(claim());
+        if (lane == 0) watch->looked = global_timer_ns();
         float length;
         const int item = now.item, s = subgrid_of(now, ranked, &length);
         if (ranked && (eager || length < kShort)) {
@@ -231,9 +233,9 @@ __device__ __forceinline__ void scout_role(const KernelArgs &a, Head *head, cons
             it.st2 = si.st2;
             it.aterm = si.aterm;
         }
-        if (k > 0) tc_wait(&head->item_free, (k - 1) & 1, abort, a.status);
+        if (k > 0) tc_wait(&head->item_free, (k - 1) & 1, watch, a.status);
         // a wait that was given up leaves the item to those who may be reading it
-        if (__any_sync(0xffffffffu, *abort)) return;
+        if (__any_sync(0xffffffffu, watch->abort)) return;
         if (lane == 0) {
             head->item = it;
             mbar_arrive(&head->item_full);
@@ -315,13 +317,13 @@ __device__ __forceinline__ void make_b(unsigned char *slot, const ChunkData &cd,
 // inputs are on their way while these are made ready.
 __device__ __forceinline__ void load_role(const KernelArgs &a, Head *head, const Layout &L, unsigned char *smem) {
     ChunkData *data = reinterpret_cast<ChunkData *>(smem + L.data);
-    volatile int *abort = &head->abort;
+    volatile TcWatch *watch = &head->watch;
     const int lane = (int)threadIdx.x - kLoadThread;
     uint32_t cn = 0; // chunks so far
     for (uint32_t k = 0;; ++k) {
-        tc_wait(&head->item_full, k & 1, abort, a.status);
+        tc_wait(&head->item_full, k & 1, watch, a.status);
         load_sync();
-        if (lane == 0) head->load_stop = head->item.stop || *abort; // one answer for all
+        if (lane == 0) head->load_stop = head->item.stop || watch->abort; // one answer for all
         load_sync();
         const Item it = head->item;
         const bool stop = head->load_stop != 0;
@@ -336,7 +338,7 @@ __device__ __forceinline__ void load_role(const KernelArgs &a, Head *head, const
         for (int chunk = 0; chunk < nchunks; ++chunk, ++cn) {
             const uint32_t buf = cn & 1;
             const int v0 = chunk * kChunk, stages = stop ? 0 : (min(it.nvis - v0, kChunk) + kStage - 1) / kStage;
-            if (cn >= 2) tc_wait(&head->c_free[buf], ((cn >> 1) - 1) & 1, abort, a.status);
+            if (cn >= 2) tc_wait(&head->c_free[buf], ((cn >> 1) - 1) & 1, watch, a.status);
             ChunkData &cd = data[buf];
             unsigned m = 0u;
 #pragma unroll 1
@@ -431,14 +433,14 @@ __device__ __forceinline__ void factor_role(const KernelArgs &a, Head *head, con
                                             uint32_t tl) {
     const float4 *axis = reinterpret_cast<const float4 *>(smem + L.axis);
     const ChunkData *data = reinterpret_cast<const ChunkData *>(smem + L.data);
-    volatile int *abort = &head->abort;
+    volatile TcWatch *watch = &head->watch;
     const int wg = threadIdx.x >> 7, warp = (threadIdx.x >> 5) & 3, t = threadIdx.x & 31, row = 8 * warp + (t >> 2);
     uint32_t turn = (uint32_t)wg, uses = 0; // stages until this warpgroup's next one; those it has done
     for (uint32_t cn = 0;; ++cn) {
         const uint32_t buf = cn & 1;
-        tc_wait(&head->c_full[buf], (cn >> 1) & 1, abort, a.status);
+        tc_wait(&head->c_full[buf], (cn >> 1) & 1, watch, a.status);
         __syncwarp();
-        if (__any_sync(0xffffffffu, *abort)) return;
+        if (__any_sync(0xffffffffu, watch->abort)) return;
         const Chunk &c = head->chunk[buf];
         if (c.stop) return;
         const uint32_t stages = (uint32_t)c.stages;
@@ -454,7 +456,7 @@ __device__ __forceinline__ void factor_role(const KernelArgs &a, Head *head, con
                 uint32_t r[2][16];
                 make_a(r, data[buf], v0 + 16 * (int)kb + 4 * (t & 3), pack2(h, h), pack2(f, f), pack2(scale, scale));
                 // the products of this warpgroup's previous half stage, and all before it, have read A and B
-                if (uses > 0 || kb > 0) tc_wait(&head->a_free[wg], (kb + 1) & 1, abort, a.status);
+                if (uses > 0 || kb > 0) tc_wait(&head->a_free[wg], (kb + 1) & 1, watch, a.status);
                 __syncwarp();
                 tmem_fence_after();
                 tmem_st_16x256_x4(tl + kColA + kColsA * wg, r[0]);
@@ -482,19 +484,19 @@ __device__ __forceinline__ void sum_role(const KernelArgs &a, Head *head, const 
                                          uint32_t tl, const Shape &sh) {
     const float2 *ntab = reinterpret_cast<const float2 *>(smem + L.ntab);
     const float4 *axis = reinterpret_cast<const float4 *>(smem + L.axis);
-    volatile int *abort = &head->abort;
+    volatile TcWatch *watch = &head->watch;
     const int lane = threadIdx.x & 127, w = lane >> 5, t = lane & 31;
     const int S = a.S, S2 = S * S, Sh = S / 2;
     unsigned char *acc = smem + L.acc;
     for (uint32_t cn = 0;; ++cn) {
         const uint32_t buf = cn & 1;
-        tc_wait(&head->c_full[buf], (cn >> 1) & 1, abort, a.status);
+        tc_wait(&head->c_full[buf], (cn >> 1) & 1, watch, a.status);
         __syncwarp();
-        if (__any_sync(0xffffffffu, *abort)) return;
+        if (__any_sync(0xffffffffu, watch->abort)) return;
         const Chunk c = head->chunk[buf];
         mbar_arrive(&head->c_free[buf]);
         if (c.stop) return;
-        tc_wait(&head->d_full[buf], (cn >> 1) & 1, abort, a.status);
+        tc_wait(&head->d_full[buf], (cn >> 1) & 1, watch, a.status);
         __syncwarp();
         tmem_fence_after();
         const f2 K = pack2(c.inv, c.inv);
@@ -599,7 +601,7 @@ __device__ __forceinline__ void issue_step(uint32_t d, uint32_t c, uint32_t k, u
 template <int XR, bool CROSS>
 __device__ __forceinline__ void issue_chunk(const KernelArgs &a, Head *head, uint32_t d, uint32_t c0, uint32_t b0,
                                             uint32_t gs, int stages, uint32_t lead) {
-    volatile int *abort = &head->abort;
+    volatile TcWatch *watch = &head->watch;
     uint32_t acc = 0;
     for (int st = 0; st < stages; st += kWorkers, gs += kWorkers) {
         const uint32_t n = (uint32_t)min(kWorkers, stages - st);
@@ -608,7 +610,7 @@ __device__ __forceinline__ void issue_chunk(const KernelArgs &a, Head *head, uin
             uint32_t w = gs % kWorkers;
 #pragma unroll 1
             for (uint32_t i = 0; i < n; ++i) {
-                tc_wait(&head->a_full[w], kb, abort, a.status); // with kb = 0, B too
+                tc_wait(&head->a_full[w], kb, watch, a.status); // with kb = 0, B too
                 tmem_fence_after();
                 if (lead) {
                     issue_step<XR, CROSS>(d, c0 + kColsA * w,
@@ -626,20 +628,20 @@ __device__ __forceinline__ void issue_chunk(const KernelArgs &a, Head *head, uin
 template <int XR>
 __device__ __forceinline__ void issue_role(const KernelArgs &a, Head *head, const Layout &L, unsigned char *smem,
                                            uint32_t tm) {
-    volatile int *abort = &head->abort;
+    volatile TcWatch *watch = &head->watch;
     const uint32_t lead = elect_lane();
     const uint32_t t0 = warp_uniform(tm), b0 = warp_uniform(umma_desc_lo(smem_addr(smem + L.b), Op<XR>::ks));
     uint32_t gs = 0;
     for (uint32_t cn = 0;; ++cn) {
         const uint32_t buf = cn & 1;
-        tc_wait(&head->c_full[buf], (cn >> 1) & 1, abort, a.status);
+        tc_wait(&head->c_full[buf], (cn >> 1) & 1, watch, a.status);
         __syncwarp();
-        if (__any_sync(0xffffffffu, *abort)) break;
+        if (__any_sync(0xffffffffu, watch->abort)) break;
         const bool stop = warp_uniform(head->chunk[buf].stop) != 0, cross = warp_uniform(head->chunk[buf].it.sg.cross) != 0;
         const int stages = (int)warp_uniform(head->chunk[buf].stages);
         mbar_arrive(&head->c_free[buf]);
         if (stop) break;
-        if (cn >= 2) tc_wait(&head->d_free[buf], ((cn >> 1) - 1) & 1, abort, a.status);
+        if (cn >= 2) tc_wait(&head->d_free[buf], ((cn >> 1) - 1) & 1, watch, a.status);
         __syncwarp();
         if (cross)
             issue_chunk<XR, true>(a, head, t0 + kColsD * buf, t0 + kColA, b0, gs, stages, lead);
@@ -684,7 +686,7 @@ __global__ void __launch_bounds__(kThreads, 1) gridder_tc_kernel(KernelArgs a) {
         mbar_init(&head->item_free, 64);
         mbar_init(&head->drain, 1);
         mbar_init_fence();
-        head->abort = 0;
+        head->watch = TcWatch{0, 0};
     }
     tc_axis_table(a, reinterpret_cast<float4 *>(smem + L.axis), sh.nb * sh.bs / 2 + 16, tid, kThreads);
     tc_n_table(a, reinterpret_cast<float2 *>(smem + L.ntab), tid, kThreads);

@@ -40,6 +40,10 @@ constexpr float kTcMaxSlope = 0.75f;     // turns of d f(x): the sincos argument
 constexpr float kTcMaxStep = 65536.f;    // turns per pixel before reduction
 constexpr double kTcMaxHalfImage = 0.12; // radians: bounds the error of c = cx cx
 constexpr uint64_t kTcWaitNs = 2000000000ull;
+// Visibilities of one item: the scout waits for as long as the item before takes,
+// at most 0.2 s in the gridder and, uncut and in four blocks, 0.6 s in the
+// degridder.  Longer subgrids go to the general kernel, whose waits are for a tile.
+constexpr int64_t kTcMaxVis = 1 << 23;
 
 // n(r2) = 1 - sqrt(1 - r2) by its series, for r2 <= 2 * 0.12^2 (next term < 1e-13).
 inline double tc_n(double r2) {
@@ -148,6 +152,7 @@ __device__ __forceinline__ void tc_offset(int X, int S, int G, float &hi, float 
 template <int NT, typename Sync>
 __device__ inline bool tc_fits(const KernelArgs &a, const SubgridInfo &si, unsigned *scratch, TcSubgrid *out,
                                Sync sync) {
+    if ((int64_t)si.T * (si.c1 - si.c0) > kTcMaxVis) return false;
     const TcConst &tc = a.tc;
     const int tid = threadIdx.x % NT, nt = NT;
     if constexpr (NT > 32) {
@@ -198,7 +203,7 @@ __device__ inline bool tc_fits(const KernelArgs &a, const SubgridInfo &si, unsig
     out->g0l = __fadd_rn(__fadd_rn(__fsub_rn(p, __fsub_rn(d, bb)), __fsub_rn(-mid, bb)), pe);
     // written so that a NaN anywhere fails
     return half * tc.eps_per_g <= kTcEps && half * tc.f_max <= kTcMaxSlope && step <= kTcMaxStep &&
-           fabsf(out->g0h) <= 1e7f && (int64_t)si.T * (si.c1 - si.c0) <= (1 << 30);
+           fabsf(out->g0h) <= 1e7f;
 }
 
 // An axis slope of one visibility in turns per pixel, off - (kh + kl) u modulo
@@ -273,14 +278,21 @@ constexpr float kTcTruncationPerStage = 1.0e-7f;
 
 // Bounded wait; on expiry raises the CTA's abort flag and the status bit, after
 // which every wait returns at once: the roles run to their next common check
-// on stale data (all addresses stay valid) and the CTA ends.
-__device__ __forceinline__ void tc_wait(uint64_t *bar, uint32_t phase, volatile int *abort, unsigned *status) {
+// on stale data (all addresses stay valid) and the CTA ends.  While the scout
+// looks at claims that it has to leave out, nothing else moves: the limit counts
+// from its last look.
+struct TcWatch {
+    uint64_t looked; // when the scout last took a claim up, ns
+    int abort;
+};
+__device__ __forceinline__ void tc_wait(uint64_t *bar, uint32_t phase, volatile TcWatch *watch, unsigned *status) {
     if (mbar_try_wait(bar, phase)) return;
     const uint64_t t0 = global_timer_ns();
     while (!mbar_try_wait(bar, phase)) {
-        if (*abort) return;
-        if (global_timer_ns() - t0 > kTcWaitNs) {
-            *abort = 1;
+        if (watch->abort) return;
+        const uint64_t now = global_timer_ns();
+        if (now - t0 > kTcWaitNs && now > watch->looked + kTcWaitNs) {
+            watch->abort = 1;
             flag_status(status, kStatusTimeout);
             return;
         }
