@@ -186,23 +186,27 @@ __device__ inline bool tc_fits(const KernelArgs &a, const SubgridInfo &si, unsig
     const float wmax = tc_unord(m[0]), wmin = -tc_unord(m[1]);
     const float kmax = tc_unord(m[2]), kmin = -tc_unord(m[3]);
     const float reach = __uint_as_float(m[4]);
-    const float g[4] = {kmin * wmin, kmin * wmax, kmax * wmin, kmax * wmax};
-    const float gmin = fminf(fminf(g[0], g[1]), fminf(g[2], g[3])) * (1.f / kTwoPiF);
-    const float gmax = fmaxf(fmaxf(g[0], g[1]), fmaxf(g[2], g[3])) * (1.f / kTwoPiF);
-    const float half = 0.5f * (gmax - gmin) * 1.0001f, mid = 0.5f * (gmax + gmin);
+    // Every operation that decides is rounded on its own: the tensor-core kernels
+    // and the general ones behind them ask this question separately, in kernels
+    // compiled separately, and a subgrid on the edge must get one answer.
+    const float g[4] = {__fmul_rn(kmin, wmin), __fmul_rn(kmin, wmax), __fmul_rn(kmax, wmin), __fmul_rn(kmax, wmax)};
+    const float gmin = __fmul_rn(fminf(fminf(g[0], g[1]), fminf(g[2], g[3])), 1.f / kTwoPiF);
+    const float gmax = __fmul_rn(fmaxf(fmaxf(g[0], g[1]), fmaxf(g[2], g[3])), 1.f / kTwoPiF);
+    const float half = __fmul_rn(0.5f * __fsub_rn(gmax, gmin), 1.0001f), mid = 0.5f * __fadd_rn(gmax, gmin);
     const float kabs = fmaxf(fabsf(kmin), fabsf(kmax));
-    const float step = kabs * reach * tc.turns_per_step;
+    const float step = __fmul_rn(__fmul_rn(kabs, reach), tc.turns_per_step);
     out->mid = mid;
-    out->cross = half * tc.eps_per_g > kTcEpsSkip;
+    const float eps = __fmul_rn(half, tc.eps_per_g);
+    out->cross = eps > kTcEpsSkip;
     tc_offset(si.X, a.S, a.G, out->xh, out->xl);
     tc_offset(si.Y, a.S, a.G, out->yh, out->yl);
     // g0 = w_step (Z + 1/2) - mid: exact product (fma), two-sum
-    const float z = (float)si.Z + 0.5f, p = __fmul_rn(a.w_step, z), pe = fmaf(a.w_step, z, -p);
+    const float z = __fadd_rn((float)si.Z, 0.5f), p = __fmul_rn(a.w_step, z), pe = fmaf(a.w_step, z, -p);
     const float d = __fsub_rn(p, mid), bb = __fsub_rn(d, p);
     out->g0h = d;
     out->g0l = __fadd_rn(__fadd_rn(__fsub_rn(p, __fsub_rn(d, bb)), __fsub_rn(-mid, bb)), pe);
     // written so that a NaN anywhere fails
-    return half * tc.eps_per_g <= kTcEps && half * tc.f_max <= kTcMaxSlope && step <= kTcMaxStep &&
+    return eps <= kTcEps && __fmul_rn(half, tc.f_max) <= kTcMaxSlope && step <= kTcMaxStep &&
            fabsf(out->g0h) <= 1e7f;
 }
 

@@ -63,3 +63,60 @@ def test_a_subgrid_too_long_for_the_bounded_waits_is_the_general_kernels(idg):
         here, general = _both(S, run)
         assert np.array_equal(here, general) and np.abs(here).max() > 0
     assert ops.device_status(clear=True) == 0
+
+
+def _edge_case(S, image_size, limit, n=3000, C=3, G=512):
+    """Subgrids of four rows whose range of w (or reach of u) steps through the
+    limit, one unit in the last place of the larger end at a time."""
+    step, edge = image_size / S, 0.5 * (S - 1) * image_size / S
+    nn = lambda r2: 1 - np.sqrt(1 - r2)
+    k = (2 * np.pi * np.linspace(150e6, 160e6, C) / 299792458.0).astype(np.float32)
+    rng = np.random.default_rng(S)
+    rows = np.zeros((n, 4, 3), np.float32)
+    rows[:, :, :2] = 40.0 * rng.standard_normal((n, 4, 2))
+    half = {"eps": 2e-3 / (2 * np.pi * (nn(2 * edge**2) - 2 * nn(edge**2))), "slope": 0.75 / nn(edge**2), "reach": 1.0}[limit]
+    w = half * 2 * np.pi / 1.0001 / float(k[-1])  # range -w .. w, the largest wavenumber
+    at = 65536.0 * 2 * np.pi / step / float(k[-1]) if limit == "reach" else w
+    ends = (np.float32(at).view(np.int32) + np.arange(n, dtype=np.int32) - n // 2).view(np.float32)
+    if limit == "reach":
+        rows[:, 2, 0] = ends
+    else:
+        rows[:, 0, 2], rows[:, 1, 2] = -ends, ends
+        rows[:, 2:, 2] = ends[:, None] * rng.uniform(-1, 1, (n, 2)).astype(np.float32)
+    md = np.zeros(n, L.METADATA_DTYPE)
+    md["time_offset"], md["nr_timesteps"], md["station2"] = 4 * np.arange(n), 4, 1
+    md["x"], md["y"] = rng.integers(0, G - S, (2, n))
+    return spec_for(G, S, C, 2, 1, image_size), md, rows.reshape(-1, 3), k
+
+
+@pytest.mark.parametrize("S", [10, 16, 24, 32, 48])
+@pytest.mark.parametrize("image_size,limit", [(0.05, "slope"), (0.15, "eps"), (0.05, "reach")])
+def test_every_subgrid_on_the_edge_of_the_rule_is_done_by_one_kernel(idg, S, image_size, limit):
+    """Outputs start as NaN; both kernels take part, so the edge is inside the range."""
+    from idg_gb300 import ops
+
+    sp, md, uvw, k = _edge_case(S, image_size, limit)
+    n, C = len(md), len(k)
+    g = torch.Generator(device="cuda")
+    g.manual_seed(S)
+    vis = torch.view_as_complex(torch.randn(4 * n, C, 4, 2, generator=g, device="cuda"))
+    sub = torch.view_as_complex(torch.randn(n, 4, S, S, 2, generator=g, device="cuda"))
+    at = torch.tensor([1, 0, 0, 1], dtype=torch.complex64, device="cuda").repeat(1, 2, S, S, 1).contiguous()
+    common, taper = (dev(md), dev(uvw), dev(k)), torch.ones(S, S, device="cuda")
+
+    def grid():
+        out = torch.full_like(sub, float("nan"))
+        ops.gridder(sp, *common, vis, taper, at, out, variant=L.VARIANT_BATCHED)
+        return out.reshape(n, -1).cpu().numpy()
+
+    def degrid():
+        out = torch.full_like(vis, float("nan"))
+        ops.degridder(sp, *common, out, taper, at, sub, variant=L.VARIANT_BATCHED)
+        return out.reshape(n, -1).cpu().numpy()
+
+    for run in (grid, degrid):
+        here, general = _both(S, run)
+        assert np.isfinite(here).all(), f"{(~np.isfinite(here).all(axis=1)).sum()} subgrids done by neither kernel"
+        same = (here == general).all(axis=1)
+        assert same.any() and not same.all()
+
