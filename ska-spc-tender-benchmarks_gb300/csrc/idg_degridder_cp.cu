@@ -637,7 +637,7 @@ __device__ __forceinline__ void column_loop_runs(f2 (&acc)[NPAIR][4][2], const K
 // UNFIT: only the subgrids that the tensor-core degridder left (tc_fits).
 template <int NT, int QB, int CB, int UNR, bool KSM, bool COL, int RUN, bool PF, bool UNFIT>
 __device__ __forceinline__ void degridder_quad_body(const KernelArgs &a) {
-    __shared__ unsigned scratch[UNFIT ? 5 : 1];
+    __shared__ unsigned scratch[UNFIT ? kTcScratch : 1];
     if (UNFIT && a.fallback[0] == 0) return;
     constexpr int kT = NT, kCB = CB, kNP = CB / 2;
     static_assert(CB == 4 || CB == 8, "channel groups of 4 or 8");

@@ -72,7 +72,7 @@ struct Head {
     TcWatch watch;
     int gen_stop;
     unsigned max_bits;
-    unsigned scratch[5];
+    unsigned scratch[kTcScratch];
     Item item;
     Job job[2];
 };

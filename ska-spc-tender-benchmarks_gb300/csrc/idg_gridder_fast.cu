@@ -405,7 +405,7 @@ __device__ __forceinline__ bool stage_tile(const KernelArgs &a, const SubgridInf
 // UNFIT: only the subgrids that the tensor-core gridder left (tc_fits).
 template <int NT, int PAIRS, int TV, int MINB, int PIPE, bool UNFIT>
 __global__ void __launch_bounds__(NT, MINB) gridder_fast_kernel(KernelArgs a) {
-    __shared__ unsigned scratch[UNFIT ? 5 : 1];
+    __shared__ unsigned scratch[UNFIT ? kTcScratch : 1];
     if (UNFIT && a.fallback[0] == 0) return;
     constexpr int kT = NT, kPairs = PAIRS, kPassPairs = NT * PAIRS, kTileVis = TV, kMaxChunk = TV;
     constexpr bool kG = (PIPE & kGauss) != 0;
@@ -711,7 +711,7 @@ __device__ __forceinline__ void quad_tile(f2 (&acc)[GP][4][8], const f2 *qg, con
 // coefficients, work distribution and failure handling as gridder_fast_kernel.
 template <int NT, int GP, int TV, int MINB, int UNR, bool UNFIT>
 __global__ void __launch_bounds__(NT, MINB) gridder_quad_kernel(KernelArgs a) {
-    __shared__ unsigned scratch[UNFIT ? 5 : 1];
+    __shared__ unsigned scratch[UNFIT ? kTcScratch : 1];
     if (UNFIT && a.fallback[0] == 0) return;
     constexpr int kT = NT, kPassQuads = NT * GP * 2, kTileVis = TV, kMaxChunk = TV;
     extern __shared__ __align__(16) unsigned char smem[];

@@ -77,7 +77,7 @@ struct Head {
     uint32_t tmem;
     TcWatch watch;
     int load_stop;
-    unsigned scratch[5];
+    unsigned scratch[kTcScratch];
     unsigned wmax[2][2];
     Item item;
     Chunk chunk[2];

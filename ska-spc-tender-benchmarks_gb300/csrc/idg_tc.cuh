@@ -145,10 +145,11 @@ __device__ __forceinline__ void tc_offset(int X, int S, int G, float &hi, float 
     lo = fmaf(-hi, q, n) / q;
 }
 
+constexpr int kTcScratch = 6;
 // Whether the expansion holds for a (valid) subgrid; NT threads (whole warps,
 // of consecutive numbers) call it and get the same answer, `sync` being their barrier.
-// `scratch`: five words of shared memory, not used by a single warp.  Only the ranges of u, v, w and of
-// the wavenumbers enter.
+// `scratch`: kTcScratch words of shared memory, not used by a single warp.  Only the
+// ranges of u, v, w and of the wavenumbers enter.
 template <int NT, typename Sync>
 __device__ inline bool tc_fits(const KernelArgs &a, const SubgridInfo &si, unsigned *scratch, TcSubgrid *out,
                                Sync sync) {
@@ -157,10 +158,12 @@ __device__ inline bool tc_fits(const KernelArgs &a, const SubgridInfo &si, unsig
     const int tid = threadIdx.x % NT, nt = NT;
     if constexpr (NT > 32) {
         sync();
-        if (tid < 5) scratch[tid] = 0u;
+        if (tid < kTcScratch) scratch[tid] = 0u;
         sync();
     }
-    unsigned m[5] = {0u, 0u, 0u, 0u, 0u}; // max of ord(w), ord(-w), ord(k), ord(-k), |u| |v| |w| as bits
+    // max of ord(w), ord(-w), ord(k), ord(-k); |u| |v| |w| and |k| as bits, which a NaN
+    // leads (its ord may be anything)
+    unsigned m[kTcScratch] = {0u, 0u, 0u, 0u, 0u, 0u};
     for (int t = tid; t < si.T; t += nt) {
         const float *p = a.uvw + 3 * ((int64_t)si.row0 + t);
         const float u = p[0], v = p[1], w = p[2];
@@ -172,20 +175,21 @@ __device__ inline bool tc_fits(const KernelArgs &a, const SubgridInfo &si, unsig
         const float k = a.wavenumbers[c];
         m[2] = max(m[2], tc_ord(k));
         m[3] = max(m[3], tc_ord(-k));
+        m[5] = max(m[5], __float_as_uint(fabsf(k)));
     }
 #pragma unroll
-    for (int i = 0; i < 5; ++i) {
+    for (int i = 0; i < kTcScratch; ++i) {
         m[i] = __reduce_max_sync(0xffffffffu, m[i]);
         if (NT > 32 && (tid & 31) == 0 && m[i]) atomicMax(&scratch[i], m[i]);
     }
     if constexpr (NT > 32) {
         sync();
 #pragma unroll
-        for (int i = 0; i < 5; ++i) m[i] = scratch[i];
+        for (int i = 0; i < kTcScratch; ++i) m[i] = scratch[i];
     }
     const float wmax = tc_unord(m[0]), wmin = -tc_unord(m[1]);
     const float kmax = tc_unord(m[2]), kmin = -tc_unord(m[3]);
-    const float reach = __uint_as_float(m[4]);
+    const float reach = __uint_as_float(m[4]), kabs = __uint_as_float(m[5]);
     // Every operation that decides is rounded on its own: the tensor-core kernels
     // and the general ones behind them ask this question separately, in kernels
     // compiled separately, and a subgrid on the edge must get one answer.
@@ -193,7 +197,6 @@ __device__ inline bool tc_fits(const KernelArgs &a, const SubgridInfo &si, unsig
     const float gmin = __fmul_rn(fminf(fminf(g[0], g[1]), fminf(g[2], g[3])), 1.f / kTwoPiF);
     const float gmax = __fmul_rn(fmaxf(fmaxf(g[0], g[1]), fmaxf(g[2], g[3])), 1.f / kTwoPiF);
     const float half = __fmul_rn(0.5f * __fsub_rn(gmax, gmin), 1.0001f), mid = 0.5f * __fadd_rn(gmax, gmin);
-    const float kabs = fmaxf(fabsf(kmin), fabsf(kmax));
     const float step = __fmul_rn(__fmul_rn(kabs, reach), tc.turns_per_step);
     out->mid = mid;
     const float eps = __fmul_rn(half, tc.eps_per_g);
@@ -205,7 +208,7 @@ __device__ inline bool tc_fits(const KernelArgs &a, const SubgridInfo &si, unsig
     const float d = __fsub_rn(p, mid), bb = __fsub_rn(d, p);
     out->g0h = d;
     out->g0l = __fadd_rn(__fadd_rn(__fsub_rn(p, __fsub_rn(d, bb)), __fsub_rn(-mid, bb)), pe);
-    // written so that a NaN anywhere fails
+    // written so that a NaN anywhere fails; one in u, v, w or k is in `step`
     return eps <= kTcEps && __fmul_rn(half, tc.f_max) <= kTcMaxSlope && step <= kTcMaxStep &&
            fabsf(out->g0h) <= 1e7f;
 }

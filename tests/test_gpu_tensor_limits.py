@@ -120,3 +120,30 @@ def test_every_subgrid_on_the_edge_of_the_rule_is_done_by_one_kernel(idg, S, ima
         same = (here == general).all(axis=1)
         assert same.any() and not same.all()
 
+
+def test_a_wavenumber_that_is_not_a_number_is_the_general_kernels(idg):
+    from idg_gb300 import ops
+
+    S, n = 32, 3
+    sp, md, uvw, k = _edge_case(S, 0.05, "slope", n=n)
+    uvw[:, 2] = 10.0
+    k[1] = np.nan
+    rng = np.random.default_rng(3)
+    vis = dev((rng.standard_normal((4 * n, 3, 4)) + 1j * rng.standard_normal((4 * n, 3, 4))).astype(np.complex64))
+    at = torch.tensor([1, 0, 0, 1], dtype=torch.complex64, device="cuda").repeat(1, 2, S, S, 1).contiguous()
+    sub = torch.ones((n, 4, S, S), dtype=torch.complex64, device="cuda")
+    args = (sp, dev(md), dev(uvw), dev(k))
+
+    def grid():
+        out = torch.zeros_like(sub)
+        ops.gridder(*args, vis, torch.ones(S, S, device="cuda"), at, out, variant=L.VARIANT_BATCHED)
+        return out.cpu().numpy()
+
+    def degrid():
+        out = torch.zeros_like(vis)
+        ops.degridder(*args, out, torch.ones(S, S, device="cuda"), at, sub, variant=L.VARIANT_BATCHED)
+        return out.cpu().numpy()
+
+    for run in (grid, degrid):
+        here, general = _both(S, run)
+        assert np.array_equal(here, general, equal_nan=True)
