@@ -59,7 +59,7 @@ struct Job {
     int stop, nc, t_begin, t_end, c0, row0, y0, add;
     int nvis;
     TcSubgrid sg;
-    float inv;
+    float inv[4]; // per polarisation
 };
 
 struct Head {
@@ -71,7 +71,7 @@ struct Head {
     uint32_t tmem;
     TcWatch watch;
     int gen_stop;
-    unsigned max_bits;
+    unsigned max_bits[4]; // per polarisation
     unsigned scratch[kTcScratch];
     Item item;
     Job job[2];
@@ -137,13 +137,14 @@ __device__ __forceinline__ void gen_sync() { named_sync<1, kGen>(); }
 __device__ __forceinline__ uint32_t op_row(int y, int p) { return (uint32_t)(16 * (y >> 2) + 4 * p + (y & 3)); }
 
 // S' of the block's pixels (x0 + x, y0 + y) into the operand layout: first the
-// largest magnitude, then scaled and split.  Returns the reciprocal scale.
+// largest magnitude of each polarisation (cross-hands may be far below the
+// others), then scaled and split.  inv: the reciprocal scales.
 // given_up: a wait ran out, perhaps one for this operand or its job; the same
 // answer for all threads.
 template <int ROWS>
-__device__ __forceinline__ float stage_block(const KernelArgs &a, const Item &si, Head *head, const Shape &sh, int x0,
+__device__ __forceinline__ void stage_block(const KernelArgs &a, const Item &si, Head *head, const Shape &sh, int x0,
                                              int y0, unsigned char *bh, const float4 *axis, const float2 *ntab,
-                                             bool *given_up) {
+                                             float (&inv)[4], bool *given_up) {
     const TcSubgrid &sg = si.sg;
     const int s = si.s;
     const int tid = threadIdx.x, S = a.S, S2 = S * S, Sh = S / 2;
@@ -155,16 +156,14 @@ __device__ __forceinline__ float stage_block(const KernelArgs &a, const Item &si
     const int kp = sh.kx / 2, items = kp * sh.nq * ROWS;
     unsigned char *bl = bh + Op<ROWS>::bytes * sh.nq, *b1 = bl + Op<ROWS>::bytes * sh.nq;
     gen_sync(); // the previous block's readers of max_bits are past it
-    if (tid == 0) {
-        head->max_bits = 0u;
-        head->gen_stop = ((volatile TcWatch *)&head->watch)->abort;
-    }
+    if (tid < 4) head->max_bits[tid] = 0u;
+    if (tid == 0) head->gen_stop = ((volatile TcWatch *)&head->watch)->abort;
     gen_sync();
     *given_up = head->gen_stop != 0;
-    if (*given_up) return 0.f;
+    if (*given_up) return;
     constexpr int kIter = 2; // at most 512 pixel pairs
     cf v[kIter][2][4];
-    unsigned m = 0u;
+    unsigned m[4] = {0u, 0u, 0u, 0u};
 #pragma unroll
     for (int it = 0; it < kIter; ++it) {
         const int i = tid + it * kGen;
@@ -192,7 +191,7 @@ __device__ __forceinline__ float stage_block(const KernelArgs &a, const Item &si
 #pragma unroll
                 for (int p = 0; p < 4; ++p) {
                     v[it][e][p] = cmul(f, v[it][e][p]);
-                    m = max(m, max(__float_as_uint(fabsf(v[it][e][p].re)), __float_as_uint(fabsf(v[it][e][p].im))));
+                    m[p] = max(m[p], max(__float_as_uint(fabsf(v[it][e][p].re)), __float_as_uint(fabsf(v[it][e][p].im))));
                 }
             } else {
 #pragma unroll
@@ -200,11 +199,15 @@ __device__ __forceinline__ float stage_block(const KernelArgs &a, const Item &si
             }
         }
     }
-    m = __reduce_max_sync(0xffffffffu, m);
-    if ((tid & 31) == 0 && m) atomicMax(&head->max_bits, m);
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+        m[p] = __reduce_max_sync(0xffffffffu, m[p]);
+        if ((tid & 31) == 0 && m[p]) atomicMax(&head->max_bits[p], m[p]);
+    }
     gen_sync();
-    float inv;
-    const float scale = tc_scale(head->max_bits, inv);
+    float scale[4];
+#pragma unroll
+    for (int p = 0; p < 4; ++p) scale[p] = tc_scale(head->max_bits[p], inv[p]);
 #pragma unroll
     for (int it = 0; it < kIter; ++it) {
         const int i = tid + it * kGen;
@@ -216,8 +219,8 @@ __device__ __forceinline__ float stage_block(const KernelArgs &a, const Item &si
         constexpr uint32_t g = ROWS * 64u; // from a row of Sr to its row of Si, and on to -Sr
 #pragma unroll
         for (int p = 0; p < 4; ++p) {
-            const f2 re = fmul2(pack2(v[it][0][p].re, v[it][1][p].re), pack2(scale, scale));
-            const f2 im = fmul2(pack2(v[it][0][p].im, v[it][1][p].im), pack2(scale, scale));
+            const f2 re = fmul2(pack2(v[it][0][p].re, v[it][1][p].re), pack2(scale[p], scale[p]));
+            const f2 im = fmul2(pack2(v[it][0][p].im, v[it][1][p].im), pack2(scale[p], scale[p]));
             uint32_t rh, rl, ih, il;
             tc_split(re, rh, rl);
             tc_split(im, ih, il);
@@ -237,7 +240,6 @@ __device__ __forceinline__ float stage_block(const KernelArgs &a, const Item &si
         }
     }
     fence_proxy_async(); // the tensor core reads the operand through the asynchronous proxy
-    return inv;
 }
 
 // x-factors of one tile into the A operand (columns Ch | Cl | Sh | Sl | A1c | A1s).
@@ -426,13 +428,14 @@ __device__ __forceinline__ void factor_role(const KernelArgs &a, Head *head, con
                 tc_wait(&head->b_free[buf], ((j >> 1) - 1) & 1, watch, a.status);
                 tc_wait(&head->job_free[buf], ((j >> 1) - 1) & 1, watch, a.status);
             }
+            float inv[4];
             bool given_up;
-            const float inv =
-                stage_block<ROWS>(a, it, head, sh, x0, y0, smem + L.b + buf * L.bset, axis, ntab, &given_up);
+            stage_block<ROWS>(a, it, head, sh, x0, y0, smem + L.b + buf * L.bset, axis, ntab, inv, &given_up);
             if (given_up) return; // the others may be reading the job that would be overwritten
             if (tid == 0)
                 head->job[buf] = Job{0, it.nc, it.t_begin, it.t_end, it.c0, it.row0, y0, block > 0, it.nvis, it.sg,
-                                     inv * kTcTruncation};
+                                     {inv[0] * kTcTruncation, inv[1] * kTcTruncation, inv[2] * kTcTruncation,
+                                      inv[3] * kTcTruncation}};
             gen_sync();
             if (tid == 0) mbar_arrive(&head->job_full[buf]);
 
@@ -541,11 +544,12 @@ __device__ __forceinline__ void result_role(const KernelArgs &a, Head *head, con
                     float o[8];
 #pragma unroll
                     for (int p = 0; p < 4; ++p) {
+                        const float inv = head->job[buf].inv[p];
                         float e, f;
                         unpack2(vr[p], e, f);
-                        o[2 * p] = (e + f) * job.inv;
+                        o[2 * p] = (e + f) * inv;
                         unpack2(vi[p], e, f);
-                        o[2 * p + 1] = (e + f) * job.inv;
+                        o[2 * p + 1] = (e + f) * inv;
                     }
                     if (job.add) {
                         // With an odd number of tiles the block before had this one in the

@@ -19,7 +19,9 @@
 //    the other warps' work.  The first-order sum's factor cx(y) is a factor of
 //    the whole row and is applied when the sum is read.
 //  * Visibilities come in chunks of 256, each scaled by a power of two to the
-//    fp16 range, and go through in stages of 32.  The tensor core truncates its
+//    fp16 range, and go through in stages of 32.  Correlations far below the
+//    others (cross-hands) have powers of their own, put in by the loading warps
+//    only then: for every chunk it would cost the 4,416 subgrids 4 %, the check 1 %.  The tensor core truncates its
 //    accumulator after every product, so the full-size and the small products
 //    have accumulators of their own and after each chunk their sum is added in
 //    fp32 to the block's sums in shared memory, while the next chunk fills the
@@ -65,7 +67,7 @@ struct Item {
 
 struct Chunk {
     int stop, stages, first, last;
-    float scale, inv;
+    float scale, inv[4]; // per polarisation
     Item it;
 };
 
@@ -78,7 +80,7 @@ struct Head {
     TcWatch watch;
     int load_stop;
     unsigned scratch[kTcScratch];
-    unsigned wmax[2][2];
+    uint4 wmax[2][2]; // per polarisation
     Item item;
     Chunk chunk[2];
 };
@@ -340,7 +342,7 @@ __device__ __forceinline__ void load_role(const KernelArgs &a, Head *head, const
             const int v0 = chunk * kChunk, stages = stop ? 0 : (min(it.nvis - v0, kChunk) + kStage - 1) / kStage;
             if (cn >= 2) tc_wait(&head->c_free[buf], ((cn >> 1) - 1) & 1, watch, a.status);
             ChunkData &cd = data[buf];
-            unsigned m = 0u;
+            unsigned m[4] = {0u, 0u, 0u, 0u};
 #pragma unroll 1
             for (int o = 0; o < stages * kStage; o += 64) {
                 const Raw r = r0;
@@ -351,7 +353,7 @@ __device__ __forceinline__ void load_role(const KernelArgs &a, Head *head, const
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
                     cd.v[i][n] = v[i];
-                    m = max(m, __float_as_uint(fabsf(v[i])));
+                    m[i >> 1] = max(m[i >> 1], __float_as_uint(fabsf(v[i])));
                 }
                 const float ph = __fmul_rn(r.k, a.tc.d2h), pl = fmaf(r.k, a.tc.d2l, fmaf(r.k, a.tc.d2h, -ph));
                 const float qh = __fmul_rn(r.k, a.tc.i2h), ql = fmaf(r.k, a.tc.i2l, fmaf(r.k, a.tc.i2h, -qh));
@@ -364,15 +366,40 @@ __device__ __forceinline__ void load_role(const KernelArgs &a, Head *head, const
                 cd.bl[n] = kTwoPiF * lo;
                 cd.d[n] = kTwoPiF * tc_delta(qh, ql, r.w, it.sg.mid);
             }
-            m = __reduce_max_sync(0xffffffffu, m);
-            if ((lane & 31) == 0) head->wmax[buf][lane >> 5] = m;
+#pragma unroll
+            for (int p = 0; p < 4; ++p) m[p] = __reduce_max_sync(0xffffffffu, m[p]);
+            if ((lane & 31) == 0) head->wmax[buf][lane >> 5] = make_uint4(m[0], m[1], m[2], m[3]);
             load_sync();
-            if (lane == 0) {
-                Chunk &c = head->chunk[buf];
+            const uint4 o = head->wmax[buf][(lane >> 5) ^ 1];
+            const unsigned w[4] = {max(m[0], o.x), max(m[1], o.y), max(m[2], o.z), max(m[3], o.w)};
+            unsigned most = 0u, least = 0xffffffffu;
+#pragma unroll
+            for (int p = 0; p < 4; ++p) {
+                most = max(most, w[p]);
+                least = min(least, w[p] - 1u); // a correlation of zeros counts as large
+            }
+            // Down to 2^-12 of the largest a correlation's lo part keeps its bits under
+            // one scale (fp16 goes down to 2^-24, 2^-36 of it).
+            const bool own = most > least && most - least > (12u << 23);
+            const auto of = [&](int p) { return p == 0 ? w[0] : p == 1 ? w[1] : p == 2 ? w[2] : w[3]; };
+            if (own && 4 * lane < stages * kStage) {
+#pragma unroll 1
+                for (int i = 0; i < 8; ++i) {
+                    float unused;
+                    const float f = tc_scale(of(i >> 1), unused);
+                    float4 &q = *reinterpret_cast<float4 *>(&cd.v[i][4 * lane]);
+                    q = make_float4(q.x * f, q.y * f, q.z * f, q.w * f);
+                }
+            }
+            Chunk &c = head->chunk[buf];
+            if (lane < 4) {
                 float inv;
-                c.scale = tc_scale(max(head->wmax[buf][0], head->wmax[buf][1]), inv);
+                const float scale = tc_scale(own ? of(lane) : most, inv);
                 // the accumulator is truncated after each of 4 products per stage: see kTcTruncation
-                c.inv = inv * (1.f + kTcTruncationPerStage * (float)stages);
+                c.inv[lane] = inv * (1.f + kTcTruncationPerStage * (float)stages);
+                if (lane == 0) c.scale = own ? 1.f : scale;
+            }
+            if (lane == 32) {
                 c.stop = stop;
                 c.stages = stages;
                 c.first = chunk == 0;
@@ -494,12 +521,13 @@ __device__ __forceinline__ void sum_role(const KernelArgs &a, Head *head, const 
         __syncwarp();
         if (__any_sync(0xffffffffu, watch->abort)) return;
         const Chunk c = head->chunk[buf];
+        const float inv = head->chunk[buf].inv[t >> 3]; // of this lane of tensor memory
         mbar_arrive(&head->c_free[buf]);
         if (c.stop) return;
         tc_wait(&head->d_full[buf], (cn >> 1) & 1, watch, a.status);
         __syncwarp();
         tmem_fence_after();
-        const f2 K = pack2(c.inv, c.inv);
+        const f2 K = pack2(inv, inv);
         const bool cross = c.it.sg.cross != 0;
         const int row = c.it.y0 + 8 * w + (t & 7); // of this lane of tensor memory
         const float4 g1 = axis[2 * (row >> 1) + 1];

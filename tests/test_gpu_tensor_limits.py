@@ -147,3 +147,30 @@ def test_a_wavenumber_that_is_not_a_number_is_the_general_kernels(idg):
     for run in (grid, degrid):
         here, general = _both(S, run)
         assert np.array_equal(here, general, equal_nan=True)
+
+
+@pytest.mark.parametrize("S", [16, 24, 32, 48])
+@pytest.mark.parametrize("faint", [1e-2, 1e-4, 1e-8, 1e-20])
+def test_a_faint_correlation_keeps_its_own_precision(oracle_mod, idg, S, faint):
+    """Correlations of very different magnitude, not mixed by the A-terms: each one by
+    itself is as close to FP64 as all of them together otherwise are (2e-6: the
+    split operands, sincos, expansion and sums of test_gpu_tensor.py)."""
+    from conftest import check_rel
+    from gpu_helpers import degrid_gpu, grid_gpu
+    from test_gpu_tensor import TOL, _case
+
+    c = _case(S, [50, 3, 17], 9, seed=S)
+    at = np.zeros_like(c["at"])
+    at[..., 0], at[..., 3] = c["at"][..., 0], c["at"][..., 3]
+    scale = np.array([1.0, faint, faint**0.5, 30.0], np.float32)
+    sp = spec_for(c["G"], S, 9, c["ns"], 1, c["img"])
+    prm = oracle_mod.params(c["G"], S, 9, c["ns"], 3, c["img"])
+    vis, sub = c["vis"] * scale, c["sub"] * scale[None, :, None, None]
+    got = grid_gpu(sp, c["md"], c["uvw"], c["k"], vis, c["taper"], at, L.VARIANT_BATCHED)
+    want = oracle_mod.gridder(prm, c["uvw"], c["k"], vis, c["taper"], at, c["md"])
+    for p in range(4):
+        check_rel(f"gridder S={S} correlation {p} of {scale[p]}", got[:, p], want[:, p], TOL)
+    got = degrid_gpu(sp, c["md"], c["uvw"], c["k"], sub, c["taper"], at, 70, L.VARIANT_BATCHED)
+    want = oracle_mod.degridder(prm, c["uvw"], c["k"], sub, c["taper"], at, c["md"], 70)
+    for p in range(4):
+        check_rel(f"degridder S={S} correlation {p} of {scale[p]}", got[..., p], want[..., p], TOL)
