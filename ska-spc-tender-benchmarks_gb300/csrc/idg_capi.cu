@@ -46,12 +46,42 @@ int current_device() {
     return dev;
 }
 
-// Degridder: the column form (32) where each lane's quads run down a column
-// for at least four steps (S a multiple of 8, S >= 32), else the row form (31).
 std::pair<int, int> default_shapes(int S) {
     const int g = S >= 8 ? gridder_fast_shapes() - 1 : general_gridder_shape(S);
     const int d = S >= 8 ? degridder_fast_shapes() - 1 : general_degridder_shape(S);
     return {g, d};
+}
+
+// Visibilities per subgrid, of n subgrids on `sms` SMs, below which the gridder
+// without tensor cores is the faster one.  The tensor-core gridder pays about 4 us
+// per subgrid and block, of one to 256 visibilities alike.  Time without over time
+// with tensor cores on GB300, 4,000 subgrids of 1, 12 and 32 visibilities:
+//   S = 12: 0.85 1.17 1.86   16: 1.08 1.26 1.67   24: 0.85 0.90 1.27   32: 1.31 1.43 1.85
+//   S = 34: 0.49 0.66 1.07   48: 0.73 0.94 1.43   56: 0.93 1.21 1.97   64: 1.17 1.36 1.64
+// With fewer the lines move: at S = 40 they cross at 28 visibilities for 8,000
+// subgrids, 23 for 2,000, 12 for 800 and nowhere for 450 (where 450 of S = 12 cross
+// at 8, of 8 and 16 at 14, in one wave of the other kernel).
+int64_t gridder_least(int S, int64_t n, int sms) {
+    if (S <= 16 && S % 8 == 0) return n > 2 * sms && n <= 4 * sms ? 12 : 0;
+    if (S <= 16) return n <= 4 * sms ? 14 : 6;
+    if (S == 24) return n > 16 * sms ? 16 : 0;
+    if (S <= 32 || S > 60) return 0;
+    if (S < 48) return n > 16 * sms ? 28 : n > 6 * sms ? 20 : n > 4 * sms ? 12 : 0;
+    if (S < 56) return n > 16 * sms ? 15 : n > 8 * sms ? 8 : 0;
+    return n > 16 * sms ? 6 : 0;
+}
+// The same for the degridder, in visibilities padded to groups of eight channels,
+// which is what the kernel without tensor cores works on.  Time ratios of 4,000
+// subgrids of 8, 256 and 384: S = 8: 0.72 0.84 1.07, 12: 0.88 1.03 1.48,
+// 16: 1.05 1.40 2.08, 20: 1.39 1.71 2.19; of 300 of 64, 256 and 512: S = 8: 0.70
+// 0.75 0.90, 12: 0.76 0.88 1.03, 16: 0.84 1.03 1.34, 20: 1.03 1.20 1.48.  With
+// fewer subgrids than SMs its tiles are shared out, two launches then cost what
+// one pass of the other kernel takes (100 of S = 16: 0.83 at 256, 1.17 at 320).
+int64_t degridder_least(int S, int64_t n, int sms) {
+    if (S <= 10) return 512;
+    if (S <= 12 || (S <= 18 && n <= sms)) return 288;
+    if (S <= 14) return n <= 4 * sms ? 192 : 64;
+    return S <= 18 && n <= 4 * sms ? 96 : 0;
 }
 
 std::pair<int, int> &shapes_of(int S) {
@@ -84,6 +114,17 @@ cudaError_t allow_dynamic_smem(const void *kernel, std::atomic<uint64_t> *done) 
     if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most - 256);
     if (e == cudaSuccess) done->fetch_or(bit, std::memory_order_release);
     return e;
+}
+
+// The mean length of a call's subgrids is that of its rows: a visibility belongs to
+// one subgrid.  (A call on some of the rows' subgrids takes them for longer.)
+bool gridder_tc_pays(const KernelArgs &a) {
+    const double n = (double)a.nr_subgrids;
+    return (double)a.nr_rows * a.C >= n * (double)gridder_least(a.S, a.nr_subgrids, launch_device().sms);
+}
+bool degridder_tc_pays(const KernelArgs &a) {
+    const double n = (double)a.nr_subgrids, padded = (double)a.nr_rows * ((a.C + 7) / 8 * 8);
+    return padded >= n * (double)degridder_least(a.S, a.nr_subgrids, launch_device().sms);
 }
 
 // Without the tensor cores: the mirror-quad gridder with 64 threads x 4 quads

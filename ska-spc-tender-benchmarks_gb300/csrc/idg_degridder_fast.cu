@@ -386,12 +386,14 @@ cudaError_t launch_shape(const KernelArgs &a, cudaStream_t stream) {
 
 // Launch shapes of the batched degridder (index = shape id).
 // Shapes 0-14 are the pixel-pair kernel above; 15 and up the channel-pair kernel.
-// The last one is the tensor-core kernel (idg_degridder_tc.cu) where it applies.
+// The last one is the tensor-core kernel (idg_degridder_tc.cu) where it applies
+// and the call's subgrids are long enough.
 int degridder_fast_shapes() { return 16 + degridder_cp_shapes(); }
 
 cudaError_t launch_degridder_fast(const KernelArgs &a, cudaStream_t stream, int shape) {
     if (shape == 15 + degridder_cp_shapes()) {
-        if (a.fallback && degridder_tc_supported(a.S, a.image_size)) return launch_degridder_tc(a, stream);
+        if (a.fallback && degridder_tc_supported(a.S, a.image_size) && degridder_tc_pays(a))
+            return launch_degridder_tc(a, stream);
         shape = general_degridder_shape(a.S);
     }
     if (shape >= 15) return launch_degridder_cp(a, stream, shape - 15);

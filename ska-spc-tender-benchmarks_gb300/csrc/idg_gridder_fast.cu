@@ -921,7 +921,8 @@ __global__ void __launch_bounds__(NT, MINB) gridder_quad_kernel(KernelArgs a) {
 //  22: shape 20 with the channel loop unrolled by four
 //  23: shape 22 with 384-visibility tiles (fewer stages per subgrid)
 //  24: shape 22 with 512-visibility tiles
-//  25: the tensor-core kernel (idg_gridder_tc.cu) where it applies, else general_gridder_shape()
+//  25: the tensor-core kernel (idg_gridder_tc.cu) where it applies and the call's
+//      subgrids are long enough, else general_gridder_shape()
 // load_only: only make sure the kernel is loaded into the current context
 // (under lazy module loading a kernel is otherwise loaded, which takes device
 // memory, at its first launch).
@@ -1001,7 +1002,8 @@ cudaError_t dispatch_gridder_fast(const KernelArgs &a, cudaStream_t stream, int 
     if (shape == 25) {
         if (load_only) return load_gridder_tc();
         // the test of a lost copy needs a kernel that stages by bulk copies
-        if (a.fallback && gridder_tc_supported(a.S, a.image_size) && !(a.flags & IDG_FLAG_TEST_LOST_COPY))
+        if (a.fallback && gridder_tc_supported(a.S, a.image_size) && gridder_tc_pays(a) &&
+            !(a.flags & IDG_FLAG_TEST_LOST_COPY))
             return launch_gridder_tc(a, stream);
         shape = general_gridder_shape(a.S);
     }

@@ -30,6 +30,7 @@ int gridder_fast_shapes();
 // Tensor-core gridder (idg_gridder_tc.cu; needs a.fallback): the subgrids its
 // expansion does not hold for go to the general kernel behind it.
 bool gridder_tc_supported(int S, double image_size);
+bool gridder_tc_pays(const KernelArgs &a); // whether the call's subgrids are long enough for it
 cudaError_t launch_gridder_tc(const KernelArgs &a, cudaStream_t stream);
 cudaError_t load_gridder_tc();
 cudaError_t launch_gridder_unfit(const KernelArgs &a, cudaStream_t stream, bool load_only);
@@ -49,6 +50,7 @@ int degridder_cp_shapes();
 // Tensor-core degridder (idg_degridder_tc.cu; needs a.fallback): the subgrids its
 // expansion does not hold for go to the general kernel behind it.
 bool degridder_tc_supported(int S, double image_size);
+bool degridder_tc_pays(const KernelArgs &a);
 cudaError_t launch_degridder_tc(const KernelArgs &a, cudaStream_t stream);
 cudaError_t launch_degridder_unfit(const KernelArgs &a, cudaStream_t stream);
 // The shape for subgrid size S among the kernels that take any geometry.

@@ -65,15 +65,15 @@ def test_a_subgrid_too_long_for_the_bounded_waits_is_the_general_kernels(idg):
     assert ops.device_status(clear=True) == 0
 
 
-def _edge_case(S, image_size, limit, n=3000, C=3, G=512):
-    """Subgrids of four rows whose range of w (or reach of u) steps through the
+def _edge_case(S, image_size, limit, n=3000, C=3, T=4, G=512):
+    """Subgrids of T rows whose range of w (or reach of u) steps through the
     limit, one unit in the last place of the larger end at a time."""
     step, edge = image_size / S, 0.5 * (S - 1) * image_size / S
     nn = lambda r2: 1 - np.sqrt(1 - r2)
     k = (2 * np.pi * np.linspace(150e6, 160e6, C) / 299792458.0).astype(np.float32)
     rng = np.random.default_rng(S)
-    rows = np.zeros((n, 4, 3), np.float32)
-    rows[:, :, :2] = 40.0 * rng.standard_normal((n, 4, 2))
+    rows = np.zeros((n, T, 3), np.float32)
+    rows[:, :, :2] = 40.0 * rng.standard_normal((n, T, 2))
     half = {"eps": 2e-3 / (2 * np.pi * (nn(2 * edge**2) - 2 * nn(edge**2))), "slope": 0.75 / nn(edge**2), "reach": 1.0}[limit]
     w = half * 2 * np.pi / 1.0001 / float(k[-1])  # range -w .. w, the largest wavenumber
     at = 65536.0 * 2 * np.pi / step / float(k[-1]) if limit == "reach" else w
@@ -82,9 +82,9 @@ def _edge_case(S, image_size, limit, n=3000, C=3, G=512):
         rows[:, 2, 0] = ends
     else:
         rows[:, 0, 2], rows[:, 1, 2] = -ends, ends
-        rows[:, 2:, 2] = ends[:, None] * rng.uniform(-1, 1, (n, 2)).astype(np.float32)
+        rows[:, 2:, 2] = ends[:, None] * rng.uniform(-1, 1, (n, T - 2)).astype(np.float32)
     md = np.zeros(n, L.METADATA_DTYPE)
-    md["time_offset"], md["nr_timesteps"], md["station2"] = 4 * np.arange(n), 4, 1
+    md["time_offset"], md["nr_timesteps"], md["station2"] = T * np.arange(n), T, 1
     md["x"], md["y"] = rng.integers(0, G - S, (2, n))
     return spec_for(G, S, C, 2, 1, image_size), md, rows.reshape(-1, 3), k
 
@@ -95,11 +95,12 @@ def test_every_subgrid_on_the_edge_of_the_rule_is_done_by_one_kernel(idg, S, ima
     """Outputs start as NaN; both kernels take part, so the edge is inside the range."""
     from idg_gb300 import ops
 
-    sp, md, uvw, k = _edge_case(S, image_size, limit)
+    T = 64 if S < 16 else 8  # long enough for the tensor-core kernels
+    sp, md, uvw, k = _edge_case(S, image_size, limit, T=T)
     n, C = len(md), len(k)
     g = torch.Generator(device="cuda")
     g.manual_seed(S)
-    vis = torch.view_as_complex(torch.randn(4 * n, C, 4, 2, generator=g, device="cuda"))
+    vis = torch.view_as_complex(torch.randn(T * n, C, 4, 2, generator=g, device="cuda"))
     sub = torch.view_as_complex(torch.randn(n, 4, S, S, 2, generator=g, device="cuda"))
     at = torch.tensor([1, 0, 0, 1], dtype=torch.complex64, device="cuda").repeat(1, 2, S, S, 1).contiguous()
     common, taper = (dev(md), dev(uvw), dev(k)), torch.ones(S, S, device="cuda")
@@ -174,3 +175,41 @@ def test_a_faint_correlation_keeps_its_own_precision(oracle_mod, idg, S, faint):
     want = oracle_mod.degridder(prm, c["uvw"], c["k"], sub, c["taper"], at, c["md"], 70)
     for p in range(4):
         check_rel(f"degridder S={S} correlation {p} of {scale[p]}", got[..., p], want[..., p], TOL)
+
+
+# (S, subgrids, steps, channels) on both sides of the lines: at S = 12 and 40 by
+# length, at 16, 24 and 48 also by the number of subgrids, and on the edges
+@pytest.mark.parametrize("S,n,T,C,grid_tc,degrid_tc", [
+    (8, 100, 3, 1, True, False), (8, 500, 11, 1, False, False), (8, 500, 12, 1, True, False), (8, 40, 64, 1, True, True),
+    (12, 600, 13, 1, False, False), (12, 600, 36, 1, True, True), (12, 50, 35, 1, True, False), (16, 100, 3, 1, True, False),
+    (16, 500, 3, 8, True, False), (16, 500, 12, 8, True, True), (16, 900, 3, 1, True, True), (14, 900, 8, 1, True, True),
+    (24, 3000, 15, 1, False, True), (24, 3000, 16, 1, True, True), (24, 900, 3, 1, True, True), (34, 4000, 27, 1, False, True),
+    (40, 300, 3, 1, True, True), (40, 1000, 10, 2, True, True), (48, 3000, 7, 2, False, True), (48, 900, 3, 1, True, True),
+    (56, 3000, 5, 1, False, True), (64, 3000, 1, 1, True, True), (32, 3000, 1, 1, True, True)])
+def test_short_subgrids_go_to_the_faster_kernel(idg, S, n, T, C, grid_tc, degrid_tc):
+    """Where the rule says so, the default shape gives the general kernel's bits."""
+    from idg_gb300 import ops
+
+    G, rng = 512, np.random.default_rng(S + n)
+    k = (2 * np.pi * np.linspace(150e6, 160e6, C) / 299792458.0).astype(np.float32)
+    md = np.zeros(n, L.METADATA_DTYPE)
+    md["time_offset"], md["nr_timesteps"], md["station2"] = T * np.arange(n), T, 1
+    md["x"], md["y"] = rng.integers(0, G - S, (2, n))
+    uvw = dev((40.0 * rng.standard_normal((T * n, 3))).astype(np.float32))
+    g = torch.Generator(device="cuda")
+    g.manual_seed(S)
+    vis = torch.view_as_complex(torch.randn(T * n, C, 4, 2, generator=g, device="cuda"))
+    sub = torch.view_as_complex(torch.randn(n, 4, S, S, 2, generator=g, device="cuda"))
+    at = torch.tensor([1, 0, 0, 1], dtype=torch.complex64, device="cuda").repeat(1, 2, S, S, 1).contiguous()
+    sp, common, taper = spec_for(G, S, C, 2, 1, 0.05), (dev(md), uvw, dev(k)), torch.ones(S, S, device="cuda")
+
+    def grid():
+        return ops.gridder(sp, *common, vis, taper, at, torch.empty_like(sub), variant=L.VARIANT_BATCHED).cpu().numpy()
+
+    def degrid():
+        return ops.degridder(sp, *common, torch.empty_like(vis), taper, at, sub, variant=L.VARIANT_BATCHED).cpu().numpy()
+
+    for run, tensor in ((grid, grid_tc), (degrid, degrid_tc)):
+        here, general = _both(S, run)
+        assert np.array_equal(here, general) != tensor
+        assert np.linalg.norm(here - general) <= 4e-6 * np.linalg.norm(general)
