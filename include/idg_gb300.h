@@ -582,7 +582,8 @@ IDG_API int idg_reference_dataset(int64_t grid_size, int64_t subgrid_size, int64
  * per SM).  Until set here or by idg_autotune(), a subgrid size uses the
  * shapes measured fastest for it on GB300 (the tensor-core kernels, the last
  * shape of each, for even sizes from 8 to 64, where a call's subgrids are long
- * enough for them; else the mirror-quad kernels where their layout fits the size).  No counterpart in the reference. */
+ * enough for them; else the mirror-quad kernels where their layout fits the
+ * size).  No counterpart in the reference. */
 IDG_API int idg_batched_shapes(int *gridder_shapes, int *degridder_shapes);
 IDG_API int idg_set_batched_shapes(int subgrid_size, int gridder_shape, int degridder_shape);
 IDG_API int idg_get_batched_shapes(int subgrid_size, int *gridder_shape, int *degridder_shape);

@@ -59,14 +59,14 @@ std::pair<int, int> default_shapes(int S) {
 //   S = 12: 0.85 1.17 1.86   16: 1.08 1.26 1.67   24: 0.85 0.90 1.27   32: 1.31 1.43 1.85
 //   S = 34: 0.49 0.66 1.07   48: 0.73 0.94 1.43   56: 0.93 1.21 1.97   64: 1.17 1.36 1.64
 // With fewer the lines move: at S = 40 they cross at 28 visibilities for 8,000
-// subgrids, 23 for 2,000, 12 for 800 and nowhere for 450 (where 450 of S = 12 cross
-// at 8, of 8 and 16 at 14, in one wave of the other kernel).
+// subgrids, 23 for 2,000, 12 for 600 and 800 and nowhere for 450 (where 450 of
+// S = 12 cross at 8, of 8 and 16 at 14, in one wave of the other kernel).
 int64_t gridder_least(int S, int64_t n, int sms) {
     if (S <= 16 && S % 8 == 0) return n > 2 * sms && n <= 4 * sms ? 12 : 0;
     if (S <= 16) return n <= 4 * sms ? 14 : 6;
     if (S == 24) return n > 16 * sms ? 16 : 0;
     if (S <= 32 || S > 60) return 0;
-    if (S < 48) return n > 16 * sms ? 28 : n > 6 * sms ? 20 : n > 4 * sms ? 12 : 0;
+    if (S < 48) return n > 16 * sms ? 28 : n > 6 * sms ? 20 : n > 3 * sms ? 12 : 0;
     if (S < 56) return n > 16 * sms ? 15 : n > 8 * sms ? 8 : 0;
     return n > 16 * sms ? 6 : 0;
 }

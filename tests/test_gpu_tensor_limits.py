@@ -184,7 +184,7 @@ def test_a_faint_correlation_keeps_its_own_precision(oracle_mod, idg, S, faint):
     (12, 600, 13, 1, False, False), (12, 600, 36, 1, True, True), (12, 50, 35, 1, True, False), (16, 100, 3, 1, True, False),
     (16, 500, 3, 8, True, False), (16, 500, 12, 8, True, True), (16, 900, 3, 1, True, True), (14, 900, 8, 1, True, True),
     (24, 3000, 15, 1, False, True), (24, 3000, 16, 1, True, True), (24, 900, 3, 1, True, True), (34, 4000, 27, 1, False, True),
-    (40, 300, 3, 1, True, True), (40, 1000, 10, 2, True, True), (48, 3000, 7, 2, False, True), (48, 900, 3, 1, True, True),
+    (40, 300, 3, 1, True, True), (40, 600, 11, 1, False, True), (40, 1000, 10, 2, True, True), (48, 3000, 7, 2, False, True), (48, 900, 3, 1, True, True),
     (56, 3000, 5, 1, False, True), (64, 3000, 1, 1, True, True), (32, 3000, 1, 1, True, True)])
 def test_short_subgrids_go_to_the_faster_kernel(idg, S, n, T, C, grid_tc, degrid_tc):
     """Where the rule says so, the default shape gives the general kernel's bits."""
