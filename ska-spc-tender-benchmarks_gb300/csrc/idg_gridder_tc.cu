@@ -128,26 +128,33 @@ __host__ __device__ inline Layout tc_layout(int S) {
 __device__ __forceinline__ void load_sync() { named_sync<1, 64>(); }
 
 // The subgrid of a claim.  More items than CTAs go longest first, or a long one
-// claimed late would be all that runs at the end: not by a sort, but the warp
+// claimed late would be all that runs at the end.  A work list is in that order
+// already and is taken as it is; otherwise not by a sort, but the warp
 // ranks 32 neighbours by their visibilities, and the claims take the longest of
 // every 32 first, then the second longest of every 32, and so on.  From the
 // first short one on, a claim and its neighbours' lengths are asked for while the
 // previous item is checked: there the scout is what the others wait for.  (With
 // long ones that would bind work to an SM too early.)  Gridding steps: 2,500
 // subgrids of 128 to 16,384 visibilities at S = 24 1.26 ms in the plan's order, 0.95
-// this way, 600 at S = 32 0.64 to 0.72 and 0.49; groups of 8 instead of 32: 1.02 and
-// 0.53.  4,416 subgrids of 128 visibilities pay 4 of 178 us for it, even ones being
-// told apart from others by one vote.
+// this way and 0.93 by a sorted list (1.29 when that was ranked once more, which
+// made 32 sweeps of it), 600 at S = 32 0.64 to 0.72, 0.43 and 0.44; groups of 8
+// instead of 32: 1.02 and 0.53.  4,416 subgrids of 128 visibilities pay 4 of 178 us
+// for it, even ones being told apart from others by one vote.
 struct Claim {
     int item, s, rank;  // work item; on each lane a neighbour of its subgrid (ranked), or that subgrid
     float length;       // the neighbour's visibilities; -1: none
 };
-__device__ __forceinline__ Claim look_up(const KernelArgs &a, int item, int nblocks, bool ranked) {
+__device__ __forceinline__ float length_of(const KernelArgs &a, int s) {
+    const int nc = a.ext ? a.ext[s].channel_end - a.ext[s].channel_begin : a.C;
+    return (float)max(a.md[s].nr_timesteps, 0) * (float)max(nc, 0);
+}
+__device__ __forceinline__ Claim look_up(const KernelArgs &a, int item, int nblocks, bool many, bool ranked) {
     Claim c{item, 0, 0, -1.f};
     const int idx = item / nblocks, n = (int)a.nr_subgrids;
     if (idx >= n) return c;
     if (!ranked) {
         c.s = a.work_list ? a.work_list[idx] : idx;
+        if (many) c.length = length_of(a, c.s);
         return c;
     }
     const int groups = (n + 31) / 32, last = n - 32 * (groups - 1); // the last group has no ranks from `last` on
@@ -156,14 +163,13 @@ __device__ __forceinline__ Claim look_up(const KernelArgs &a, int item, int nblo
     const int group = late < 0 ? idx - c.rank * groups : late - (c.rank - last) * (groups - 1);
     const int i = 32 * group + (int)(threadIdx.x & 31);
     if (i < n) {
-        c.s = a.work_list ? a.work_list[i] : i;
-        const int nc = a.ext ? a.ext[c.s].channel_end - a.ext[c.s].channel_begin : a.C;
-        c.length = (float)max(a.md[c.s].nr_timesteps, 0) * (float)max(nc, 0);
+        c.s = i;
+        c.length = length_of(a, i);
     }
     return c;
 }
 __device__ __forceinline__ int subgrid_of(const Claim &c, bool ranked, float *length) {
-    *length = 0.f;
+    *length = c.length;
     if (!ranked) return c.s;
     const float first = __shfl_sync(0xffffffffu, c.length, 0);
     int who = c.rank;
@@ -187,9 +193,9 @@ __device__ __forceinline__ void scout_role(const KernelArgs &a, Head *head, cons
     volatile TcWatch *watch = &head->watch;
     const int lane = threadIdx.x & 31, nblocks = sh.nb * sh.nb, S2 = a.S * a.S;
     const size_t jones = (size_t)S2 * 2;
-    const bool ranked = a.nr_subgrids * nblocks > (int64_t)gridDim.x;
+    const bool many = a.nr_subgrids * nblocks > (int64_t)gridDim.x, ranked = many && !a.work_list;
     auto claim = [&] { return lane > 0 ? 0 : watch->abort ? INT32_MAX : atomicAdd(a.work_counter, 1); };
-    auto look = [&](int c) { return look_up(a, __shfl_sync(0xffffffffu, c, 0), nblocks, ranked); };
+    auto look = [&](int c) { return look_up(a, __shfl_sync(0xffffffffu, c, 0), nblocks, many, ranked); };
     Claim next{};
     int ahead = 0;      // the claim after the next one
     bool eager = false; // down to the short ones
@@ -198,7 +204,7 @@ __device__ __forceinline__ void scout_role(const KernelArgs &a, Head *head, cons
         if (lane == 0) watch->looked = global_timer_ns();
         float length;
         const int item = now.item, s = subgrid_of(now, ranked, &length);
-        if (ranked && (eager || length < kShort)) {
+        if (many && (eager || length < kShort)) {
             next = look(eager ? ahead : claim());
             ahead = claim();
             eager = true;

@@ -213,3 +213,33 @@ def test_short_subgrids_go_to_the_faster_kernel(idg, S, n, T, C, grid_tc, degrid
         here, general = _both(S, run)
         assert np.array_equal(here, general) != tensor
         assert np.linalg.norm(here - general) <= 4e-6 * np.linalg.norm(general)
+
+
+@pytest.mark.parametrize("S,n", [(24, 400), (32, 153), (48, 100)])
+def test_a_plans_work_list_is_taken_as_it_is(idg, S, n):
+    """A plan's list is longest first and every subgrid in it once: the same bits as the
+    separate steps, which take the subgrids in another order."""
+    from idg_gb300 import ops
+    from test_gpu_tensor import _case
+
+    rng = np.random.default_rng(n)
+    lengths = [int(x) for x in rng.choice([0, 1, 9, 40, 40, 200, 400], n)]
+    lengths[3] = 40
+    c = _case(S, lengths, 9, seed=n)
+    rows = slice(int(c["md"]["time_offset"][3]), int(c["md"]["time_offset"][3]) + 40)
+    c["uvw"][rows, 2] += (8000.0 * np.sin(np.arange(40))).astype(np.float32)  # left to the general kernel
+    data = [dev(c[k]) for k in ("uvw", "k", "vis", "taper", "at")]
+    grids = [torch.zeros((1, 4, c["G"], c["G"]), dtype=torch.complex64, device="cuda") for _ in range(2)]
+    sp = spec_for(c["G"], S, 9, c["ns"], 1, c["img"])
+    plan = ops.Plan(sp, c["md"], c["uvw"].shape[0])
+    plan.grid(*data, grids[0])
+    sub = torch.empty((n, 4, S, S), dtype=torch.complex64, device="cuda")
+    ops.gridder(spec_for(c["G"], S, 9, c["ns"], 1, c["img"], flags=L.IDG_FLAG_NO_TAPER), dev(c["md"]), *data[:3], None,
+                data[4], sub, variant=L.VARIANT_BATCHED)
+    ops.subgrid_fft(sp, sub, 1, data[3])
+    bins = ops.TileBins(sp, c["md"])
+    bins.add(sub, grids[1])
+    assert torch.equal(torch.view_as_real(grids[0]), torch.view_as_real(grids[1])) and grids[0].abs().max() > 0
+    assert plan.status() == 0
+    bins.close()
+    plan.close()
