@@ -116,6 +116,17 @@ cudaError_t allow_dynamic_smem(const void *kernel, std::atomic<uint64_t> *done) 
     return e;
 }
 
+cudaError_t resident_ctas(const void *kernel, int threads, size_t smem, std::atomic<uint64_t> *known, int *ctas) {
+    const uint64_t k = known->load(std::memory_order_relaxed);
+    *ctas = (int)(k & 0xff);
+    if (*ctas > 0 && k >> 8 == smem) return cudaSuccess;
+    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(ctas, kernel, threads, smem);
+    if (e != cudaSuccess) return e;
+    if (*ctas < 1) *ctas = 1;
+    known->store((uint64_t)smem << 8 | (uint64_t)*ctas, std::memory_order_relaxed);
+    return cudaSuccess;
+}
+
 // The mean length of a call's subgrids is that of its rows: a visibility belongs to
 // one subgrid.  (A call on some of the rows' subgrids takes them for longer.)
 bool gridder_tc_pays(const KernelArgs &a) {

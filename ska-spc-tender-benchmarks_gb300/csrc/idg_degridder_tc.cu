@@ -373,6 +373,10 @@ __device__ __forceinline__ void scout_role(const KernelArgs &a, int nseg, Head *
             }
             const int nc = si.c1 - si.c0;
             if (nc == 0 || si.T == 0) continue;
+            if (!tc_fits<32>(a, si, head->scratch, &it.sg, [] { __syncwarp(); })) {
+                if (lane == 0) atomicAdd(a.fallback, 1);
+                continue;
+            }
             const char *px = reinterpret_cast<const char *>(a.subgrids + (size_t)sj * 4 * a.S * a.S);
             const char *j1 = reinterpret_cast<const char *>(a.aterms + ((size_t)si.aterm * a.nr_stations + si.st1) * jones);
             const char *j2 = reinterpret_cast<const char *>(a.aterms + ((size_t)si.aterm * a.nr_stations + si.st2) * jones);
@@ -380,10 +384,6 @@ __device__ __forceinline__ void scout_role(const KernelArgs &a, int nseg, Head *
                 asm volatile("prefetch.global.L2 [%0];" ::"l"(px + o));
                 asm volatile("prefetch.global.L2 [%0];" ::"l"(j1 + o));
                 asm volatile("prefetch.global.L2 [%0];" ::"l"(j2 + o));
-            }
-            if (!tc_fits<32>(a, si, head->scratch, &it.sg, [] { __syncwarp(); })) {
-                if (lane == 0) atomicAdd(a.fallback, 1);
-                continue;
             }
             it.s = sj;
             it.row0 = si.row0;

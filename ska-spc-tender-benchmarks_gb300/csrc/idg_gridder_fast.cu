@@ -936,11 +936,14 @@ cudaError_t launch_shape(const KernelArgs &a, cudaStream_t stream, bool load_onl
     const size_t smem = layout(a.S, a.C, TV).total;
     int64_t blocks = 0;
     cudaError_t e;
-    if constexpr (UNFIT) { // usually nothing to do: no queries
+    if constexpr (UNFIT) { // usually nothing to do: no queries but the first
         static std::atomic<uint64_t> allowed{0};
         e = allow_dynamic_smem(reinterpret_cast<const void *>(kern), &allowed);
         if (e != cudaSuccess) return e;
-        blocks = (int64_t)launch_device().sms * MINB;
+        static std::atomic<uint64_t> known{0};
+        int per_sm = 0;
+        if ((e = resident_ctas(reinterpret_cast<const void *>(kern), NT, smem, &known, &per_sm)) != cudaSuccess) return e;
+        blocks = (int64_t)launch_device().sms * per_sm;
     } else {
         e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
@@ -970,11 +973,14 @@ cudaError_t launch_quad(const KernelArgs &a, cudaStream_t stream, bool load_only
     const size_t smem = quad_layout(a.C, TV).total + (size_t)NT * GP * 3 * sizeof(f2); // + quad geometry
     int64_t blocks = 0;
     cudaError_t e;
-    if constexpr (UNFIT) { // usually nothing to do: no queries
+    if constexpr (UNFIT) { // usually nothing to do: no queries but the first
         static std::atomic<uint64_t> allowed{0};
         e = allow_dynamic_smem(reinterpret_cast<const void *>(kern), &allowed);
         if (e != cudaSuccess) return e;
-        blocks = (int64_t)launch_device().sms * MINB;
+        static std::atomic<uint64_t> known{0};
+        int per_sm = 0;
+        if ((e = resident_ctas(reinterpret_cast<const void *>(kern), NT, smem, &known, &per_sm)) != cudaSuccess) return e;
+        blocks = (int64_t)launch_device().sms * per_sm;
     } else {
         e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;

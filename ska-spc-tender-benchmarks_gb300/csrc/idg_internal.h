@@ -19,6 +19,9 @@ struct LaunchDevice {
 };
 LaunchDevice launch_device();
 cudaError_t allow_dynamic_smem(const void *kernel, std::atomic<uint64_t> *done);
+// CTAs of a kernel that an SM holds at once, at least 1.  `known`: a static of the
+// caller, one per kernel, that remembers the answer for the last amount of shared memory.
+cudaError_t resident_ctas(const void *kernel, int threads, size_t smem, std::atomic<uint64_t> *known, int *ctas);
 
 // IDG_VARIANT_PLAIN: one CTA per subgrid (idg_gridder.cu / idg_degridder.cu).
 // IDG_VARIANT_BATCHED: persistent packed-FP32x2 kernels (idg_*_fast.cu); need a.work_counter.
