@@ -1,9 +1,11 @@
 // idg_server.cu -- the serving loop: continuous batching of gridding and
 // degridding jobs on one GPU.
 //
-// Jobs arrive on any thread through idg_server_submit().  A scheduler thread
-// admits them in arrival order whenever a slot (a CUDA stream) is free and the
-// job's device footprint fits the HBM budget left by the jobs already running
+// Jobs arrive on any thread through idg_server_submit(), which works out all it can
+// and leaves them in an inbox without waiting for the scheduler: that keeps its
+// lock while it copies pageable inputs in, and takes the next job up right after.
+// A scheduler thread admits them in arrival order whenever a slot (a CUDA stream)
+// is free and the job's device footprint fits the HBM budget left by the jobs already running
 // -- a job that can never fit is rejected at submission.  An admitted job gets
 // one stream-ordered allocation for its plan, subgrid work space and data, its
 // copies in, the batched kernels of its step and its copies out, all on its
@@ -75,6 +77,7 @@ struct Job {
     double dev_start_ms = -1, dev_end_ms = -1; // k0, k1 relative to the server's epoch event
     double work_start_ms = -1, work_end_ms = -1; // c0, c1
     double est_ms = 0;                      // estimated device time at the full CTA budget
+    bool copy_out_left = false;             // the results are copied out once the kernels have ended
     int share = 1;                          // its kernels' share of that budget: 1 / share
     int status = IDG_OK;
     bool finished = false;
@@ -115,20 +118,29 @@ struct idg_server {
     idg_server_config cfg{};
     int device = 0;
     std::mutex mu;
-    std::condition_variable cv_work, cv_done;
+    std::condition_variable cv_done;
     std::deque<std::shared_ptr<Job>> queue;
+    // Submitted jobs that the scheduler has not taken up yet.  Locks are taken in the
+    // order mu, grids_mu, inbox_mu.
+    std::mutex inbox_mu;
+    std::condition_variable cv_work; // with inbox_mu
+    std::vector<std::shared_ptr<Job>> inbox;
+    int64_t next_job = 1; // with inbox_mu
+    bool woken = false;   // with inbox_mu
     std::map<int64_t, std::shared_ptr<Job>> jobs;
     std::vector<std::shared_ptr<Job>> slots;
     std::vector<cudaStream_t> streams;
     cudaEvent_t epoch = nullptr; // recorded at creation: origin of the jobs' device intervals
     std::map<int64_t, Grid> grids;
-    int64_t next_job = 1, next_grid = 1;
+    mutable std::mutex grids_mu; // held beside mu where grids come and go: submissions look them up without mu
+    int64_t next_grid = 1;
     size_t in_use = 0, peak_use = 0;
     // device milliseconds per 1e9 pixel-visibilities of a job's kernels at the
     // full CTA budget: a running estimate from the finished jobs (seeded with
     // GB300's config-2 rate)
     double ms_per_gpv = 0.6;
-    int64_t completed = 0, rejected = 0, failed = 0, total_vis = 0;
+    int64_t completed = 0, failed = 0, total_vis = 0;
+    std::atomic<int64_t> rejected{0};
     std::vector<double> latencies;
     Clock::time_point first_submit{}, last_done{};
     bool have_first = false;
@@ -136,12 +148,22 @@ struct idg_server {
     std::thread worker;
 
     void run();
+    void wake();
+    int64_t take_inbox_locked(); // returns the last job's number
     void admit_locked();
     void launch(Job &j);
+    void copy_out(Job &j);
     void poll_locked();
 };
 
 namespace {
+
+bool pageable(const void *host) {
+    cudaPointerAttributes at{};
+    if (cudaPointerGetAttributes(&at, host) == cudaSuccess) return at.type == cudaMemoryTypeUnregistered;
+    cudaGetLastError();
+    return true;
+}
 
 int validate_job(const idg_server *srv, const idg_job *j) {
     if (!j) return fail(IDG_ERR_INVALID_ARGUMENT, "job is NULL");
@@ -153,10 +175,13 @@ int validate_job(const idg_server *srv, const idg_job *j) {
         return fail(IDG_ERR_INVALID_ARGUMENT, "NULL host array");
     if (j->op == IDG_JOB_GRID && !j->vis_in) return fail(IDG_ERR_INVALID_ARGUMENT, "gridding job without vis_in");
     if (j->op == IDG_JOB_DEGRID && !j->vis_out) return fail(IDG_ERR_INVALID_ARGUMENT, "degridding job without vis_out");
-    auto it = srv->grids.find(j->grid_id);
-    if (it == srv->grids.end()) return fail(IDG_ERR_NOT_FOUND, "unknown grid %lld", (long long)j->grid_id);
-    if (it->second.size != j->params.grid_size || it->second.planes != (j->params.nr_w_planes > 0 ? j->params.nr_w_planes : 1))
-        return fail(IDG_ERR_INVALID_ARGUMENT, "job geometry does not match grid %lld", (long long)j->grid_id);
+    {
+        std::lock_guard<std::mutex> lock(srv->grids_mu);
+        auto it = srv->grids.find(j->grid_id);
+        if (it == srv->grids.end()) return fail(IDG_ERR_NOT_FOUND, "unknown grid %lld", (long long)j->grid_id);
+        if (it->second.size != j->params.grid_size || it->second.planes != (j->params.nr_w_planes > 0 ? j->params.nr_w_planes : 1))
+            return fail(IDG_ERR_INVALID_ARGUMENT, "job geometry does not match grid %lld", (long long)j->grid_id);
+    }
     const int bo1 = j->metadata[0].baseline_offset;
     for (int64_t s = 0; s < j->nr_subgrids; ++s) {
         const idg_metadata &m = j->metadata[s];
@@ -175,6 +200,18 @@ int validate_job(const idg_server *srv, const idg_job *j) {
 }
 
 } // namespace
+
+// A degridding job's results, on its stream; the end of its stream work.
+void idg_server::copy_out(Job &j) {
+    const idg_job &spec = j.spec;
+    cudaError_t e = cudaSuccess;
+    if (spec.op == IDG_JOB_DEGRID)
+        e = cudaMemcpyAsync(spec.vis_out, static_cast<char *>(j.arena) + job_layout(spec).vis,
+                            (size_t)spec.nr_rows * spec.params.nr_channels * 32, cudaMemcpyDeviceToHost, streams[j.slot]);
+    if (e == cudaSuccess && j.c1) e = cudaEventRecord(j.c1, streams[j.slot]);
+    if (e != cudaSuccess && j.status == IDG_OK) j.status = cuda_fail(e, "server job copy out");
+    j.copy_out_left = false;
+}
 
 void idg_server::launch(Job &j) {
     cudaSetDevice(device);
@@ -289,10 +326,12 @@ void idg_server::launch(Job &j) {
         chk(launch_degridder(a, variant, p.nr_channels, st));
     }
     if (j.k1) chk(cudaEventRecord(j.k1, st));
-    if (j.spec.op == IDG_JOB_DEGRID)
-        chk(cudaMemcpyAsync(j.spec.vis_out, dp(L.vis), b_vis, cudaMemcpyDeviceToHost, st));
-    if (j.c1) chk(cudaEventRecord(j.c1, st));
-    chk(cudaEventRecord(j.done, st));
+    // A copy to pageable memory holds this thread until the kernels before it have
+    // ended.  With jobs waiting it is left for then, so that the next one's kernels
+    // run beside this one's.
+    j.copy_out_left = j.spec.op == IDG_JOB_DEGRID && queue.size() > 1 && pageable(j.spec.vis_out);
+    if (!j.copy_out_left) copy_out(j);
+    chk(cudaEventRecord(j.done, st)); // the job needs its grid no longer
     if (g.last_op != j.spec.op) g.holders.clear();
     g.last_op = j.spec.op;
     g.holders.push_back(j.done);
@@ -304,13 +343,9 @@ void idg_server::admit_locked() {
     std::vector<int64_t> blocked;
     auto is_blocked = [&](int64_t g) { return std::find(blocked.begin(), blocked.end(), g) != blocked.end(); };
     for (auto it = queue.begin(); it != queue.end();) {
-        int free_slot = -1;
-        for (int s = 0; s < (int)slots.size(); ++s)
-            if (!slots[s]) {
-                free_slot = s;
-                break;
-            }
-        if (free_slot < 0) return;
+        const auto free_at = std::find(slots.begin(), slots.end(), nullptr);
+        if (free_at == slots.end()) return;
+        const int free_slot = (int)(free_at - slots.begin());
         Job &j = **it;
         // a gridding job must not change a grid while idg_server_grid_read copies it out
         const bool grid_being_read = j.spec.op == IDG_JOB_GRID && grids[j.spec.grid_id].readers > 0;
@@ -350,7 +385,11 @@ void idg_server::admit_locked() {
             j.c0 = j.c1 = nullptr; // ... and without its stream interval
         }
         launch(j);
-        it = queue.erase(it);
+        const auto at = it - queue.begin();
+        queue.erase(it);
+        take_inbox_locked(); // jobs that came during the copies
+        poll_locked();       // and those that ended
+        it = queue.begin() + at;
         cv_done.notify_all(); // a grid read may be waiting for this job's admission
     }
 }
@@ -366,6 +405,10 @@ void idg_server::poll_locked() {
         cudaError_t q = cudaStreamQuery(streams[s]);
         if (q == cudaErrorNotReady) continue;
         Job &j = *jp;
+        if (j.copy_out_left && q == cudaSuccess && j.status == IDG_OK) {
+            copy_out(j);
+            if ((q = cudaStreamQuery(streams[s])) == cudaErrorNotReady) continue;
+        }
         j.t_done = Clock::now();
         if (q != cudaSuccess && j.status == IDG_OK) j.status = cuda_fail(q, "server job");
         if (j.k0 && j.k1 && q == cudaSuccess && j.status == IDG_OK) {
@@ -431,18 +474,43 @@ void idg_server::poll_locked() {
     }
 }
 
+void idg_server::wake() {
+    {
+        std::lock_guard<std::mutex> lock(inbox_mu);
+        woken = true;
+    }
+    cv_work.notify_all();
+}
+
+int64_t idg_server::take_inbox_locked() {
+    std::lock_guard<std::mutex> lock(inbox_mu);
+    for (auto &j : inbox) {
+        if (!have_first) first_submit = j->t_submit;
+        have_first = true;
+        jobs[j->id] = j;
+        queue.push_back(std::move(j));
+    }
+    inbox.clear();
+    return next_job - 1;
+}
+
 void idg_server::run() {
     cudaSetDevice(device);
-    std::unique_lock<std::mutex> lock(mu);
     for (;;) {
-        poll_locked();
-        admit_locked();
         bool running = false;
-        for (auto &s : slots)
-            if (s) running = true;
-        if (stop && !running && queue.empty()) break;
+        {
+            std::lock_guard<std::mutex> lock(mu);
+            take_inbox_locked();
+            poll_locked();
+            admit_locked();
+            for (auto &s : slots)
+                if (s) running = true;
+            if (stop && !running && queue.empty()) break;
+        }
         // short sleep while kernels run; wake at once on new work
-        cv_work.wait_for(lock, std::chrono::microseconds(running ? 100 : 2000));
+        std::unique_lock<std::mutex> lock(inbox_mu);
+        cv_work.wait_for(lock, std::chrono::microseconds(running ? 100 : 2000), [&] { return woken || !inbox.empty(); });
+        woken = false;
     }
 }
 
@@ -505,7 +573,7 @@ IDG_API int idg_server_destroy(idg_server *srv) {
         std::lock_guard<std::mutex> lock(srv->mu);
         srv->stop = true;
     }
-    srv->cv_work.notify_all();
+    srv->wake();
     srv->worker.join();
     cudaSetDevice(srv->device);
     for (auto &g : srv->grids) cudaFree(g.second.dev);
@@ -526,6 +594,7 @@ IDG_API int idg_server_grid_create(idg_server *srv, int32_t grid_size, int32_t n
     IDG_CUDA(cudaMalloc(&g.dev, g.bytes));
     IDG_CUDA(cudaMemset(g.dev, 0, g.bytes));
     std::lock_guard<std::mutex> lock(srv->mu);
+    std::lock_guard<std::mutex> grids_lock(srv->grids_mu);
     *grid_id = srv->next_grid++;
     srv->grids[*grid_id] = g;
     return IDG_OK;
@@ -547,7 +616,7 @@ IDG_API int idg_server_grid_read(idg_server *srv, int64_t grid_id, void *host_ou
     size_t bytes = 0;
     {
         std::unique_lock<std::mutex> lock(srv->mu);
-        const int64_t last_job = srv->next_job - 1;
+        const int64_t last_job = srv->take_inbox_locked();
         auto queued_before = [&] {
             for (auto &q : srv->queue)
                 if (q->spec.grid_id == grid_id && q->id <= last_job) return true;
@@ -582,7 +651,7 @@ IDG_API int idg_server_grid_read(idg_server *srv, int64_t grid_id, void *host_ou
         std::lock_guard<std::mutex> lock(srv->mu);
         --srv->grids[grid_id].readers;
     }
-    srv->cv_work.notify_all(); // gridding jobs held back by the read may start
+    srv->wake(); // gridding jobs held back by the read may start
     if (e != cudaSuccess) return cuda_fail(e, "grid read");
     return IDG_OK;
 }
@@ -590,6 +659,8 @@ IDG_API int idg_server_grid_read(idg_server *srv, int64_t grid_id, void *host_ou
 IDG_API int idg_server_grid_release(idg_server *srv, int64_t grid_id) {
     if (!srv) return fail(IDG_ERR_INVALID_ARGUMENT, "NULL server");
     std::lock_guard<std::mutex> lock(srv->mu);
+    std::lock_guard<std::mutex> grids_lock(srv->grids_mu); // from here on no new job finds the grid
+    srv->take_inbox_locked();
     auto it = srv->grids.find(grid_id);
     if (it == srv->grids.end()) return fail(IDG_ERR_NOT_FOUND, "unknown grid %lld", (long long)grid_id);
     if (!it->second.holders.empty()) return fail(IDG_ERR_REJECTED, "grid %lld has jobs in flight", (long long)grid_id);
@@ -605,10 +676,7 @@ IDG_API int idg_server_grid_release(idg_server *srv, int64_t grid_id) {
 IDG_API int idg_server_submit(idg_server *srv, const idg_job *job, int64_t *job_id) {
     if (!srv || !job_id) return fail(IDG_ERR_INVALID_ARGUMENT, "NULL argument");
     auto j = std::make_shared<Job>();
-    {
-        std::lock_guard<std::mutex> lock(srv->mu);
-        if (int rc = validate_job(srv, job)) return rc;
-    }
+    if (int rc = validate_job(srv, job)) return rc;
     j->spec = *job;
     const int64_t N = job->nr_subgrids;
     j->md.assign(job->metadata, job->metadata + N);
@@ -625,21 +693,21 @@ IDG_API int idg_server_submit(idg_server *srv, const idg_job *job, int64_t *job_
     if (job->op == IDG_JOB_GRID)
         if (int rc = bin_tiles(&job->params, N, job->metadata, &j->bins)) return rc;
     j->footprint = job_layout(j->spec, job->op == IDG_JOB_GRID ? &j->bins : nullptr).total;
-    std::lock_guard<std::mutex> lock(srv->mu);
     if (j->footprint > (size_t)srv->cfg.hbm_budget_bytes) {
         ++srv->rejected;
         return fail(IDG_ERR_REJECTED, "job needs %zu bytes of device memory, the budget is %lld", j->footprint,
                     (long long)srv->cfg.hbm_budget_bytes);
     }
-    j->id = srv->next_job++;
-    j->t_submit = Clock::now();
-    if (!srv->have_first) {
-        srv->first_submit = j->t_submit;
-        srv->have_first = true;
+    {
+        std::lock_guard<std::mutex> grids_lock(srv->grids_mu);
+        if (srv->grids.find(job->grid_id) == srv->grids.end()) // released meanwhile
+            return fail(IDG_ERR_NOT_FOUND, "unknown grid %lld", (long long)job->grid_id);
+        std::lock_guard<std::mutex> lock(srv->inbox_mu);
+        j->id = srv->next_job++;
+        j->t_submit = Clock::now();
+        *job_id = j->id;
+        srv->inbox.push_back(std::move(j));
     }
-    srv->jobs[j->id] = j;
-    srv->queue.push_back(j);
-    *job_id = j->id;
     srv->cv_work.notify_all();
     return IDG_OK;
 }
@@ -647,6 +715,7 @@ IDG_API int idg_server_submit(idg_server *srv, const idg_job *job, int64_t *job_
 IDG_API int idg_server_wait(idg_server *srv, int64_t job_id, int64_t timeout_ms, idg_job_stats *stats) {
     if (!srv) return fail(IDG_ERR_INVALID_ARGUMENT, "NULL server");
     std::unique_lock<std::mutex> lock(srv->mu);
+    srv->take_inbox_locked();
     auto it = srv->jobs.find(job_id);
     if (it == srv->jobs.end()) return fail(IDG_ERR_NOT_FOUND, "unknown job %lld", (long long)job_id);
     std::shared_ptr<Job> j = it->second;
@@ -673,6 +742,7 @@ IDG_API int idg_server_stats(idg_server *srv, idg_server_summary *out) {
     if (!srv || !out) return fail(IDG_ERR_INVALID_ARGUMENT, "NULL argument");
     std::lock_guard<std::mutex> lock(srv->mu);
     memset(out, 0, sizeof *out);
+    srv->take_inbox_locked();
     out->completed = srv->completed;
     out->rejected = srv->rejected;
     out->failed = srv->failed;
