@@ -136,9 +136,11 @@ struct idg_server {
     int64_t next_grid = 1;
     size_t in_use = 0, peak_use = 0;
     // device milliseconds per 1e9 pixel-visibilities of a job's kernels at the
-    // full CTA budget: a running estimate from the finished jobs (seeded with
-    // GB300's config-2 rate)
-    double ms_per_gpv = 0.6;
+    // full CTA budget: a running estimate from the finished jobs.  It starts at the
+    // rate of either step of the benchmark observation on GB300 (664e9 in 86.7 ms):
+    // too high a start takes finished peers for running ones, and jobs get a half
+    // or a third of the SMs for it.
+    double ms_per_gpv = 0.13;
     int64_t completed = 0, failed = 0, total_vis = 0;
     std::atomic<int64_t> rejected{0};
     std::vector<double> latencies;
