@@ -66,8 +66,11 @@ def get_shapes(subgrid_size: int) -> tuple[int, int]:
 
 
 def apply_cached(spec: GridSpec) -> dict | None:
-    """Select the cached shapes for this device / subgrid size / channel count, if any."""
+    """Select the cached shapes for this device / subgrid size / channel count, if any.
+    A choice made among other shapes than the library now has does not count."""
     entry = _load().get(_key(spec))
+    if entry and (len(entry.get("gridder_ms", ())), len(entry.get("degridder_ms", ()))) != num_shapes():
+        return None
     if entry:
         set_shapes(spec.subgrid_size, int(entry["gridder"]), int(entry["degridder"]))
     return entry
