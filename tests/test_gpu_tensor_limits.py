@@ -243,3 +243,26 @@ def test_a_plans_work_list_is_taken_as_it_is(idg, S, n):
     assert plan.status() == 0
     bins.close()
     plan.close()
+
+
+@pytest.mark.parametrize("S", [16, 32, 48])
+def test_edges_of_the_gridders_chunks(oracle_mod, idg, S):
+    """A chunk holds 256 visibilities: one below, at and above one and two of them."""
+    from test_gpu_tensor import TOL, _case, _degrid, _grid
+
+    c = _case(S, [255, 256, 257, 512, 513], 1, seed=S)
+    _grid(c, oracle_mod, f"S={S} chunk edges", TOL)
+    _degrid(c, oracle_mod, f"S={S} chunk edges", TOL)
+
+
+@pytest.mark.parametrize("chunk", [0, 1, 2, 3])
+def test_every_chunk_has_a_scale_of_its_own(oracle_mod, idg, chunk):
+    """Four chunks of very different magnitude, all but one of them zero: its own
+    contribution is as exact as any."""
+    from test_gpu_tensor import TOL, _case, _grid
+
+    c = _case(32, [256], 4, seed=12)
+    keep = np.zeros(256, np.float32)
+    keep[64 * chunk:64 * chunk + 64] = 10.0 ** (6 * chunk - 9)
+    c["vis"] *= keep[:, None, None]
+    _grid(c, oracle_mod, f"chunk {chunk}", TOL)
