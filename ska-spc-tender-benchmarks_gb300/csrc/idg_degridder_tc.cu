@@ -59,7 +59,7 @@ struct Job {
     int stop, nc, t_begin, t_end, c0, row0, y0, add;
     int nvis;
     TcSubgrid sg;
-    float inv[4]; // per polarisation
+    float4 inv; // per polarisation
 };
 
 struct Head {
@@ -71,7 +71,7 @@ struct Head {
     uint32_t tmem;
     TcWatch watch;
     int gen_stop;
-    unsigned max_bits[4]; // per polarisation
+    uint4 max_bits; // per polarisation
     unsigned scratch[kTcScratch];
     Item item;
     Job job[2];
@@ -144,7 +144,7 @@ __device__ __forceinline__ uint32_t op_row(int y, int p) { return (uint32_t)(16 
 template <int ROWS>
 __device__ __forceinline__ void stage_block(const KernelArgs &a, const Item &si, Head *head, const Shape &sh, int x0,
                                              int y0, unsigned char *bh, const float4 *axis, const float2 *ntab,
-                                             float (&inv)[4], bool *given_up) {
+                                             float4 &inv, bool *given_up) {
     const TcSubgrid &sg = si.sg;
     const int s = si.s;
     const int tid = threadIdx.x, S = a.S, S2 = S * S, Sh = S / 2;
@@ -156,7 +156,7 @@ __device__ __forceinline__ void stage_block(const KernelArgs &a, const Item &si,
     const int kp = sh.kx / 2, items = kp * sh.nq * ROWS;
     unsigned char *bl = bh + Op<ROWS>::bytes * sh.nq, *b1 = bl + Op<ROWS>::bytes * sh.nq;
     gen_sync(); // the previous block's readers of max_bits are past it
-    if (tid < 4) head->max_bits[tid] = 0u;
+    if (tid < 4) (&head->max_bits.x)[tid] = 0u;
     if (tid == 0) head->gen_stop = ((volatile TcWatch *)&head->watch)->abort;
     gen_sync();
     *given_up = head->gen_stop != 0;
@@ -200,14 +200,11 @@ __device__ __forceinline__ void stage_block(const KernelArgs &a, const Item &si,
         }
     }
 #pragma unroll
-    for (int p = 0; p < 4; ++p) {
-        m[p] = __reduce_max_sync(0xffffffffu, m[p]);
-        if ((tid & 31) == 0 && m[p]) atomicMax(&head->max_bits[p], m[p]);
-    }
+    for (int p = 0; p < 4; ++p) m[p] = __reduce_max_sync(0xffffffffu, m[p]);
+    if ((tid & 31) < 4) atomicMax(&head->max_bits.x + (tid & 3), (tid & 2) ? (tid & 1) ? m[3] : m[2] : (tid & 1) ? m[1] : m[0]);
     gen_sync();
-    float scale[4];
-#pragma unroll
-    for (int p = 0; p < 4; ++p) scale[p] = tc_scale(head->max_bits[p], inv[p]);
+    const uint4 most = head->max_bits;
+    const float scale[4] = {tc_scale(most.x, inv.x), tc_scale(most.y, inv.y), tc_scale(most.z, inv.z), tc_scale(most.w, inv.w)};
 #pragma unroll
     for (int it = 0; it < kIter; ++it) {
         const int i = tid + it * kGen;
@@ -428,14 +425,14 @@ __device__ __forceinline__ void factor_role(const KernelArgs &a, Head *head, con
                 tc_wait(&head->b_free[buf], ((j >> 1) - 1) & 1, watch, a.status);
                 tc_wait(&head->job_free[buf], ((j >> 1) - 1) & 1, watch, a.status);
             }
-            float inv[4];
+            float4 inv;
             bool given_up;
             stage_block<ROWS>(a, it, head, sh, x0, y0, smem + L.b + buf * L.bset, axis, ntab, inv, &given_up);
             if (given_up) return; // the others may be reading the job that would be overwritten
             if (tid == 0)
                 head->job[buf] = Job{0, it.nc, it.t_begin, it.t_end, it.c0, it.row0, y0, block > 0, it.nvis, it.sg,
-                                     {inv[0] * kTcTruncation, inv[1] * kTcTruncation, inv[2] * kTcTruncation,
-                                      inv[3] * kTcTruncation}};
+                                     make_float4(inv.x * kTcTruncation, inv.y * kTcTruncation, inv.z * kTcTruncation,
+                                                 inv.w * kTcTruncation)};
             gen_sync();
             if (tid == 0) mbar_arrive(&head->job_full[buf]);
 
@@ -541,10 +538,11 @@ __device__ __forceinline__ void result_role(const KernelArgs &a, Head *head, con
                 if (i < nvis) {
                     const int t = i / job.nc, c = job.c0 + i - t * job.nc;
                     float4 *dst = a.vis + (((int64_t)job.row0 + t) * a.C + c) * 2;
+                    const float4 i4 = head->job[buf].inv;
                     float o[8];
 #pragma unroll
                     for (int p = 0; p < 4; ++p) {
-                        const float inv = head->job[buf].inv[p];
+                        const float inv = p == 0 ? i4.x : p == 1 ? i4.y : p == 2 ? i4.z : i4.w;
                         float e, f;
                         unpack2(vr[p], e, f);
                         o[2 * p] = (e + f) * inv;
