@@ -139,12 +139,10 @@ __device__ __forceinline__ uint32_t op_row(int y, int p) { return (uint32_t)(16 
 // S' of the block's pixels (x0 + x, y0 + y) into the operand layout: first the
 // largest magnitude of each polarisation (cross-hands may be far below the
 // others), then scaled and split.  inv: the reciprocal scales.
-// given_up: a wait ran out, perhaps one for this operand or its job; the same
-// answer for all threads.
 template <int ROWS>
 __device__ __forceinline__ void stage_block(const KernelArgs &a, const Item &si, Head *head, const Shape &sh, int x0,
                                              int y0, unsigned char *bh, const float4 *axis, const float2 *ntab,
-                                             float4 &inv, bool *given_up) {
+                                             float4 &inv) {
     const TcSubgrid &sg = si.sg;
     const int s = si.s;
     const int tid = threadIdx.x, S = a.S, S2 = S * S, Sh = S / 2;
@@ -157,10 +155,7 @@ __device__ __forceinline__ void stage_block(const KernelArgs &a, const Item &si,
     unsigned char *bl = bh + Op<ROWS>::bytes * sh.nq, *b1 = bl + Op<ROWS>::bytes * sh.nq;
     gen_sync(); // the previous block's readers of max_bits are past it
     if (tid < 4) (&head->max_bits.x)[tid] = 0u;
-    if (tid == 0) head->gen_stop = ((volatile TcWatch *)&head->watch)->abort;
     gen_sync();
-    *given_up = head->gen_stop != 0;
-    if (*given_up) return;
     constexpr int kIter = 2; // at most 512 pixel pairs
     cf v[kIter][2][4];
     unsigned m[4] = {0u, 0u, 0u, 0u};
@@ -399,7 +394,7 @@ __device__ __forceinline__ void scout_role(const KernelArgs &a, int nseg, Head *
 }
 
 // Factor warps: subgrid after subgrid, its staging, then this warpgroup's tiles.
-template <int ROWS>
+template <int ROWS, bool BLOCKS>
 __device__ __forceinline__ void factor_role(const KernelArgs &a, Head *head, const Shape &sh, const Layout &L,
                                             unsigned char *smem, uint32_t tl) {
     const float4 *axis = reinterpret_cast<const float4 *>(smem + L.axis);
@@ -418,18 +413,16 @@ __device__ __forceinline__ void factor_role(const KernelArgs &a, Head *head, con
         mbar_arrive(&head->item_free);
         if (stop) break;
 
-        for (int block = 0; block < sh.nb * sh.nb; ++block, ++j) {
-            const int x0 = (block % sh.nb) * sh.bs, y0 = (block / sh.nb) * sh.bs;
+        for (int block = 0; block < (BLOCKS ? 4 : 1); ++block, ++j) {
+            const int x0 = (block & 1) * sh.bs, y0 = (block >> 1) * sh.bs;
             const uint32_t buf = j & 1;
             if (j >= 2) {
                 tc_wait(&head->b_free[buf], ((j >> 1) - 1) & 1, watch, a.status);
                 tc_wait(&head->job_free[buf], ((j >> 1) - 1) & 1, watch, a.status);
             }
             float4 inv;
-            bool given_up;
-            stage_block<ROWS>(a, it, head, sh, x0, y0, smem + L.b + buf * L.bset, axis, ntab, inv, &given_up);
-            if (given_up) return; // the others may be reading the job that would be overwritten
-            if (tid == 0)
+            stage_block<ROWS>(a, it, head, sh, x0, y0, smem + L.b + buf * L.bset, axis, ntab, inv);
+            if (tid == 0 && !watch->abort) // after a wait that was given up others may be reading the last one
                 head->job[buf] = Job{0, it.nc, it.t_begin, it.t_end, it.c0, it.row0, y0, block > 0, it.nvis, it.sg,
                                      make_float4(inv.x * kTcTruncation, inv.y * kTcTruncation, inv.z * kTcTruncation,
                                                  inv.w * kTcTruncation)};
@@ -469,7 +462,7 @@ __device__ __forceinline__ void factor_role(const KernelArgs &a, Head *head, con
 }
 
 // Result warps: H times the y-factors, summed over the rows.
-template <int ROWS>
+template <int ROWS, bool BLOCKS>
 __device__ __forceinline__ void result_role(const KernelArgs &a, Head *head, const Shape &sh, const Layout &L,
                                             unsigned char *smem, uint32_t tl) {
     const float4 *axis = reinterpret_cast<const float4 *>(smem + L.axis);
@@ -484,6 +477,11 @@ __device__ __forceinline__ void result_role(const KernelArgs &a, Head *head, con
         if (__any_sync(0xffffffffu, watch->abort)) return;
         const Job job = head->job[buf];
         if (job.stop) return;
+        // With an odd number of tiles the block before had a tile in the other
+        // warpgroup: its stores come before this one's reads.  (Its threads are past that
+        // job or ahead of this one in the products' order, so they never wait for this
+        // one.)
+        if (BLOCKS && job.add) tc_wait(&head->job_free[buf ^ 1], ((j - 1) >> 1) & 1, watch, a.status);
         const int nvis = job.nvis;
         const uint32_t n0 = n;
         int tile = job.t_begin + (int)((n ^ (uint32_t)wg) & 1u);
@@ -549,12 +547,7 @@ __device__ __forceinline__ void result_role(const KernelArgs &a, Head *head, con
                         unpack2(vi[p], e, f);
                         o[2 * p + 1] = (e + f) * inv;
                     }
-                    if (job.add) {
-                        // With an odd number of tiles the block before had this one in the
-                        // other warpgroup: its stores come first.  (Its threads are past that
-                        // job or ahead of this one in the products' order, so they never wait
-                        // for this one.)
-                        tc_wait(&head->job_free[buf ^ 1], ((j - 1) >> 1) & 1, watch, a.status);
+                    if (BLOCKS && job.add) {
                         const float4 e = dst[0], f = dst[1];
                         o[0] += e.x, o[1] += e.y, o[2] += e.z, o[3] += e.w;
                         o[4] += f.x, o[5] += f.y, o[6] += f.z, o[7] += f.w;
@@ -631,7 +624,8 @@ __device__ __forceinline__ void issue_role(const KernelArgs &a, Head *head, cons
     __syncwarp();
 }
 
-template <int ROWS>
+// BLOCKS: subgrids larger than 32, in four blocks.
+template <int ROWS, bool BLOCKS>
 __global__ void __launch_bounds__(kThreads, 1) degridder_tc_kernel(KernelArgs a, int nseg) {
     extern __shared__ __align__(128) unsigned char smem[];
     const Shape sh = tc_shape(a.S);
@@ -671,9 +665,9 @@ __global__ void __launch_bounds__(kThreads, 1) degridder_tc_kernel(KernelArgs a,
     const uint32_t tl = tm + ((uint32_t)(warp & 3) << 21); // this warp's lane quarter
 
     if (warp < 8)
-        factor_role<ROWS>(a, head, sh, L, smem, tl);
+        factor_role<ROWS, BLOCKS>(a, head, sh, L, smem, tl);
     else if (warp < 16)
-        result_role<ROWS>(a, head, sh, L, smem, tl);
+        result_role<ROWS, BLOCKS>(a, head, sh, L, smem, tl);
     else if (warp == 16)
         issue_role<ROWS>(a, head, sh, L, smem, tm);
     else
@@ -682,9 +676,9 @@ __global__ void __launch_bounds__(kThreads, 1) degridder_tc_kernel(KernelArgs a,
     if (warp == 16) tmem_free(tm, kTmemCols);
 }
 
-template <int ROWS>
+template <int ROWS, bool BLOCKS>
 cudaError_t launch(const KernelArgs &args, cudaStream_t stream) {
-    auto kern = degridder_tc_kernel<ROWS>;
+    auto kern = degridder_tc_kernel<ROWS, BLOCKS>;
     KernelArgs a = args;
     a.tc = tc_const(a.S, a.image_size);
     const size_t smem = tc_layout<ROWS>(a.S, a.C).total;
@@ -709,10 +703,11 @@ bool degridder_tc_supported(int S, double image_size) {
 }
 
 cudaError_t launch_degridder_tc(const KernelArgs &a, cudaStream_t stream) {
+    const bool blocks = a.S > 32;
     switch (tc_shape(a.S).rows) {
-    case 8: return launch<8>(a, stream);
-    case 12: return launch<12>(a, stream);
-    default: return launch<16>(a, stream);
+    case 8: return launch<8, false>(a, stream); // S = 8
+    case 12: return blocks ? launch<12, true>(a, stream) : launch<12, false>(a, stream);
+    default: return blocks ? launch<16, true>(a, stream) : launch<16, false>(a, stream);
     }
 }
 
