@@ -627,8 +627,9 @@ def run_ours(args, rank, world, local_rank):
                           "subgrids of this shape, scaled by subgrids (the kernels stream each subgrid's data once)",
         "peak_source": "tensor: " + tensor_source + " (fp16 runs at the bf16 rate); fp32: measured in this run, FFMA "
                        "microbenchmark idg_measure_fp32_peak",
-        "algorithmic": "tensor: three fp16 products for the 32 flop of four complex MACs, 96 flop per pixel-visibility; "
-                       "fp32: 34 flop (17 FMA) + 1 sincos; %.3g pixel-visibilities per launch" % pixvis,
+        "algorithmic": "tensor: the algorithm needs 32 flop (four complex MACs) per pixel-visibility, this form executes 96 "
+                       "(three fp16 products), counted in `achieved`; fp32: 34 flop (17 FMA) + 1 sincos; %.3g "
+                       "pixel-visibilities per launch" % pixvis,
         "peak_check": peak_check,
         "gridder": per_kernel["gridder"],
         "degridder": per_kernel["degridder"],
@@ -720,7 +721,8 @@ def run_ours(args, rank, world, local_rank):
         "higher_is_better": True,
         "scaling": "weak",
         "vs_baseline": None,
-        "dtype": "f32 (FP64 per-subgrid phase offsets)",
+        "dtype": ("f32 in and out; products of fp16 hi + lo pairs summed in f32, phases in f32 pairs" if all(tensor)
+                  else "f32 (FP64 per-subgrid phase offsets)"),
         "data": "synthetic (seeded; N(0,1) visibilities, earth-rotation uvw)",
         "config": config_block(spec, args.workload, {"variant": args.variant, "parallelism": f"replicas x{world}",
                                                      "tuned_shapes": tune}),

@@ -116,8 +116,8 @@ IDG_API const char *idg_last_error(void);
 /* Reads and (if clear != 0) resets the device-side check word of the current
  * device: bit 0 = a plan entry named rows/stations/A-terms out of range,
  * bit 1 = a shape the kernel cannot handle, bit 2 = a staged copy did not
- * arrive within its time limit (the kernel stopped; its outputs are
- * incomplete).  Synchronises `stream`. */
+ * arrive, or a role of a tensor-core kernel did not hear from another, within
+ * the time limit (the kernel stopped; its outputs are incomplete).  Synchronises `stream`. */
 IDG_API int idg_device_status(void *stream, uint32_t *status, int clear);
 
 /* ------------------------------------------------------------------ */
