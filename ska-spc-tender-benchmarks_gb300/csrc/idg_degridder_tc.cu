@@ -22,8 +22,9 @@
 //    its pixels and A-terms; the factor warps, which have time to spare, stage
 //    its S' into the other of two buffers while the tensor core works on the
 //    current one.
-// One CTA of 18 warps per SM: 448 columns of tensor memory, 147 KB of operands.
-// Measured on GB300, 4,416 subgrids of 128 x 16 visibilities at S = 32: 0.87 ms
+// One CTA of 18 warps per SM: all of its tensor memory (448 of the 512 columns that
+// an allocation has to be are used), 147 KB of operands.
+// Measured on GB300, 4,416 subgrids of 128 x 16 visibilities at S = 32: 0.90 ms
 // (24.6 SM cycles per visibility beyond a fixed 7 us per subgrid and SM), against
 // 5.27 ms for the mirror-quad kernel.  The products alone take 16 cycles per
 // visibility; the rest is the issue slots of the factor and result warps, which

@@ -21,17 +21,17 @@
 //  * Visibilities come in chunks of 256, each scaled by a power of two to the
 //    fp16 range, and go through in stages of 32.  Correlations far below the
 //    others (cross-hands) have powers of their own, put in by the loading warps
-//    only then: for every chunk it would cost the 4,416 subgrids 4 %, the check 1 %.  The tensor core truncates its
-//    accumulator after every product, so the full-size and the small products
-//    have accumulators of their own and after each chunk their sum is added in
-//    fp32 to the block's sums in shared memory, while the next chunk fills the
-//    other buffer.
+//    only then: for every chunk it would cost the 4,416 subgrids 4 %, the check 1 %.
+//    The tensor core truncates its accumulator after every product, so the
+//    full-size and the small products have accumulators of their own and after
+//    each chunk their sum is added in fp32 to the block's sums in shared memory,
+//    while the next chunk fills the other buffer.
 //  * Roles: four factor warpgroups that take stages in turn, both operands of
 //    one (an own half stage of A, an own stage of B each); a fifth for the sums
 //    and the epilogue; two warps that bring in the chunks, one that issues the
 //    products, one that looks for the next subgrid.
 // One CTA of 24 warps per SM and all of its tensor memory.
-// Measured on GB300, 4,416 subgrids of 128 x 16 visibilities at S = 32: 1.26 ms
+// Measured on GB300, 4,416 subgrids of 128 x 16 visibilities at S = 32: 1.27 ms
 // (41 SM cycles per visibility) against 5.02 ms for the mirror-quad kernel.  The
 // products take 16 of those cycles.  The rest is the traffic of factors between
 // the roles: with the factors' arithmetic left out, or the loads, or the stores,
@@ -42,7 +42,7 @@
 // instead of a predicate on each.  The roles run five different loops on one SM,
 // so these are kept small: with the half stages unrolled and two stages of
 // x-factors at a time, the same work missed the instruction cache (1.47 ms).
-// 28 subgrids of 64 x 16 in one call: 39 us against 213 us.
+// 28 subgrids of 64 x 16 in one call: 40 us against 213 us.
 #include "idg_tc.cuh"
 #include "idg_internal.h"
 

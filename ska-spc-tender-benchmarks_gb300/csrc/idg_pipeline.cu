@@ -63,8 +63,10 @@ struct Chunk {
 // whose sizes grow by `ratio` from one to the next (`growing`) or shrink by
 // it (otherwise), chunks under a quarter of the plan, but at least 512 and at most
 // kMinChunk subgrids, merged into their neighbour; anything else: one chunk.
-// (Chunks of 512: a cycle of 2,016 subgrids takes 2.08 ms in two chunks, 2.21 in
-// one, 2.22 in four; 8,010 take 5.20 in four of 1,024 or more, 5.27 in five.)  A
+// (Chunks of 512: a cycle of 2,016 subgrids takes 2.07 ms in two chunks, 2.21 in
+// one, 2.22 in four; 8,010 take 5.20 in four of 1,024 or more, 5.27 in five.  Against
+// at least 1,024 for every plan, cycles of 1,540 and 2,556 take 1.81 and 2.32 ms, not
+// 1.90 and 2.55; 780, 1,081, 1,225, 3,003, 4,005 and 5,995 the same.)  A
 // growing chunk's copy keeps ahead of the previous chunk's kernels while the copy
 // rate is at least `ratio` times the rate the kernels consume visibilities (the
 // gridder takes about 180 GB/s at S = 32).

@@ -51,7 +51,7 @@ constexpr int kChunk = 128;     // subgrids per pass-1 work item (at most 256: t
 // for (8,000 subgrids of 32^2 spread over 4096^2: 490 us, this way 330, with the
 // cells in registers 353; over 2048^2 185, 136 and 144).
 // Measured on GB300, 9,180 subgrids of 32^2 added to a cleared 2048^2 grid (20 us of
-// clearing included): 107 us, where one CTA per item with every warp going
+// clearing included): 105 us, where one CTA per item with every warp going
 // through all entries, two rows 16 apart per thread, took 157 (73 % of the issue
 // slots busy, half of them with cells outside the footprint); with two
 // neighbouring rows per warp 115.  365 MB are read, 54 us at the copy rate; 412
