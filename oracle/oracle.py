@@ -31,10 +31,13 @@ REF_DEGRIDDER_CUBIN = os.path.join(HERE, "_ref", "ref_degridder.cubin")
 def _reference_dir() -> str:
     """Where the reference sources are: $IDG_REFERENCE_DIR when set, else the
     default that oracle/Makefile (the recipe that compiles them) gives
-    IDG_REFERENCE_DIR; empty when neither names one."""
-    env = os.environ.get("IDG_REFERENCE_DIR", "")
-    if env:
-        return env
+    IDG_REFERENCE_DIR; empty when neither names one, or the one named holds no
+    gridding sources."""
+    found = os.environ.get("IDG_REFERENCE_DIR", "") or _makefile_dir()
+    return found if os.path.isdir(os.path.join(found, "gridding", "src")) else ""
+
+
+def _makefile_dir() -> str:
     try:
         with open(os.path.join(HERE, "Makefile")) as f:
             for line in f:
